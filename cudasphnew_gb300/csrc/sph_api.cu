@@ -58,6 +58,8 @@ void* host_device_ptr(const void* p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
+RowMasks masks_of(const sph_sim* s) { return RowMasks{s->rowStart, s->rowMask}; }
+
 RowTables rows_of(const sph_sim* s) {
     return RowTables{s->sb.cellOffset, s->sb.halfOffset, s->sb.scenes, s->sb.skip};
 }
@@ -122,7 +124,7 @@ sph_status validate_params(const SimulationParameters* P, const sph_options* O) 
     if (O && (O->cellRelative < 0 || O->cellRelative > 1))
         SPH_FAIL(SPH_ERR_INVALID_ARGUMENT, "cellRelative must be 0 or 1");
     // at most 0.4: the skin sphere then spans at most 4 cells per axis (compactSupport <= gridSpacing),
-    // so a particle's rows fit the lists' VL_SLOTS = 16 entries
+    // so a particle has at most VL_ROWS = 16 rows
     if (O && !(O->neighbourSkin >= 0.0f && O->neighbourSkin <= 0.4f))
         SPH_FAIL(SPH_ERR_INVALID_ARGUMENT, "neighbourSkin must be in [0, 0.4]");
     if (O && O->cellRelative &&
@@ -171,7 +173,7 @@ void free_all(sph_sim* s) {
                     s->sb.keySlot, s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds,
                     s->sb.halfOffset, s->scanBlock,
                     s->status, s->staging, s->map4, s->mapDist, s->rowStart, s->rowMask, s->diagBuf,
-                    s->scenesDev, s->reuse, s->vl.start, s->vl.skin, s->vl.exact, s->vl.rows, s->vl.posB,
+                    s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.posB,
                     s->vl.flags, s->vl.slotScene};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -302,10 +304,8 @@ sph_status alloc_lists(sph_sim* s) {
     if (!(s->O.neighbourSkin > 0.0f) || s->O.cellRelative) return SPH_OK;
     const size_t n = (size_t)s->n;
     const int S = std::max(s->numScenes, 1);
-    SPH_CUDA(dalloc(&s->vl.start, VL_SLOTS * n));
-    SPH_CUDA(dalloc(&s->vl.skin, VL_SLOTS * n));
-    SPH_CUDA(dalloc(&s->vl.exact, VL_SLOTS * n));
-    SPH_CUDA(dalloc(&s->vl.rows, n));
+    SPH_CUDA(dalloc(&s->vl.list, VL_GROUPS * n));
+    SPH_CUDA(dalloc(&s->vl.groups, n));
     SPH_CUDA(dalloc(&s->vl.posB, n));
     SPH_CUDA(dalloc(&s->vl.flags, (size_t)VL_FLAGS * S + VL_GLOBAL));
     SPH_CUDA(cudaMemsetAsync(s->vl.flags, 0, sizeof(unsigned int) * (VL_FLAGS * S + VL_GLOBAL), s->stream));
@@ -317,7 +317,8 @@ sph_status alloc_lists(sph_sim* s) {
         SPH_CUDA(dalloc(&s->vl.slotScene, n));
         SPH_CUDA(cudaMemcpy(s->vl.slotScene, scene.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     }
-    SPH_CUDA(cudaMemsetAsync(s->vl.rows, 0, n, s->stream));
+    SPH_CUDA(cudaMemsetAsync(s->vl.groups, 0, n, s->stream));
+    launch_list_far_record((int)n, s->posS, s->velS, s->stream);
     set_list_radius(s);
     s->vlOn = true;
     request_list_build(s);
@@ -344,12 +345,13 @@ static void enqueue_lists(sph_sim* s, const GridDev& g, const PhysDev& ph, int c
     mark(ST_RANK);
     launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, &s->vl, s->status);
     mark(ST_DENSITY);
-    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, s->cfg, true, true, st);
+    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, true,
+                         true, st);
     // the sorted copies are now this step's own: a reuse the audit granted is used up
     cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
     mark(ST_FORCE);
-    launch_force_lists(n, s->posS, s->velS, s->rho4S, s->sb.workIds, ph, s->map, collide, s->vl, s->pos, s->vel,
-                       s->accS, s->cfg, st, s->sb.scenes);
+    launch_force_lists(n, s->posS, s->velS, s->rho4S, s->sb.workIds, ph, s->map, collide, s->vl, masks_of(s), s->pos,
+                       s->vel, s->accS, s->cfg, st, s->sb.scenes);
     mark(ST_FORCE + 1);  // the force stage's end
     s->lastStepLists = true;
 }
@@ -412,7 +414,8 @@ void enqueue_list_density(sph_sim* s, const float4* pos, const float4* vel) {
     launch_cell_scan(g.numCells, s->sb, s->status, st, &s->vl);
     launch_scatter(n, s->sb, st, s->status, &s->vl);
     launch_rank_gather(n, s->sb, pos, vel, g, s->posS, s->velS, st, &s->vl, s->status);
-    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, s->cfg, true, true, st);
+    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, true,
+                         true, st);
 }
 
 void invalidate_graphs(sph_sim* s) {
@@ -497,8 +500,8 @@ sph_status alloc_handle(sph_sim* s, int n, long long C) {
     s->stream = s->ownStream;
     SPH_CUDA(dalloc(&s->pos, n));
     SPH_CUDA(dalloc(&s->vel, n));
-    SPH_CUDA(dalloc(&s->posS, n));
-    SPH_CUDA(dalloc(&s->velS, n));
+    SPH_CUDA(dalloc(&s->posS, (size_t)n + 1));  // [n]: the lists' far record
+    SPH_CUDA(dalloc(&s->velS, (size_t)n + 1));
     SPH_CUDA(dalloc(&s->rho4S, n));
     SPH_CUDA(dalloc(&s->accS, n));
     SPH_CUDA(dalloc(&s->rowStart, (size_t)9 * n));
@@ -1330,10 +1333,8 @@ static sph_status autotune_lists(sph_sim* s, int reps, sph_tuning* chosen) {
                 {s->sb.workIds, nullptr, sizeof(int) * n},      {s->sb.cellOffset, nullptr, sizeof(int) * C1},
                 {s->sb.halfOffset, nullptr, sizeof(int) * C1},
                 {s->vl.flags, nullptr, sizeof(unsigned int) * (VL_FLAGS * s->vl.numScenes + VL_GLOBAL)},
-                {s->vl.start, nullptr, sizeof(int) * VL_SLOTS * n},
-                {s->vl.skin, nullptr, sizeof(uint2) * VL_SLOTS * n},
-                {s->vl.exact, nullptr, sizeof(uint2) * VL_SLOTS * n},
-                {s->vl.rows, nullptr, (size_t)n},               {s->vl.posB, nullptr, sizeof(float4) * n}};
+                {s->vl.list, nullptr, sizeof(int4) * VL_GROUPS * n},
+                {s->vl.groups, nullptr, (size_t)n},             {s->vl.posB, nullptr, sizeof(float4) * n}};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto cleanup = [&]() {
         for (auto& b : bufs)
@@ -1612,20 +1613,46 @@ sph_status sph_time_kernel(sph_handle s, int stage, int reps, float* microsecond
     // the density stage rewrites what it wrote (and the masks the force form
     // reads); the force stage rewrites the state the last step wrote
     SPH_CUDA(cudaMemsetAsync(s->reuse, 0, sizeof(int), st));
-    // after a step over the reused neighbour lists the list forms are timed
-    // (the density stage's list form: the lists match the sorted copies)
+    // after a step over the reused neighbour lists the list forms are timed,
+    // also where that step built them (the lists match the sorted copies); what
+    // the launches write is kept and put back, since a building step's sums
+    // are taken in another order
     const bool lists = s->vlOn && s->lastStepLists;
-    if (lists)
-        SPH_CUDA(cudaMemsetAsync(s->vl.flags + VL_BUILD_NOW * s->vl.numScenes, 0,
-                                 sizeof(unsigned int) * s->vl.numScenes, st));
+    struct Kept {
+        void* at;
+        size_t bytes;
+        void* copy;
+    } kept[] = {{s->pos, sizeof(float4) * n, nullptr},   {s->vel, sizeof(float4) * n, nullptr},
+                {s->accS, sizeof(float4) * n, nullptr},  {s->rho4S, sizeof(float4) * n, nullptr},
+                {s->posS, sizeof(float4) * n, nullptr},  {s->velS, sizeof(float4) * n, nullptr},
+                {s->vl.flags, sizeof(unsigned int) * (VL_FLAGS * s->vl.numScenes + VL_GLOBAL), nullptr}};
+    auto forget = [&]() {
+        for (Kept& k : kept)
+            if (k.copy) cudaFree(k.copy);
+    };
+    if (lists) {
+        cudaError_t e = cudaSuccess;
+        for (Kept& k : kept) {
+            if (e == cudaSuccess) e = cudaMalloc(&k.copy, k.bytes);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(k.copy, k.at, k.bytes, cudaMemcpyDeviceToDevice, st);
+        }
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(s->vl.flags + VL_BUILD_NOW * s->vl.numScenes, 0,
+                                sizeof(unsigned int) * s->vl.numScenes, st);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(st);
+            forget();
+            SPH_CUDA(e);
+        }
+    }
     auto launch = [&]() {
         if (lists) {
             if (stage == ST_DENSITY)
-                launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, s->cfg, false, true,
-                                     st);
+                launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg,
+                                     false, true, st);
             else
                 launch_force_lists(n, s->posS, s->velS, s->rho4S, s->sb.workIds, ph, s->map, s->O.boxCollision,
-                                   s->vl, s->pos, s->vel, s->accS, s->cfg, st, s->sb.scenes);
+                                   s->vl, masks_of(s), s->pos, s->vel, s->accS, s->cfg, st, s->sb.scenes);
         } else if (stage == ST_DENSITY) {
             launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, s->cfg, st);
         } else {
@@ -1634,17 +1661,12 @@ sph_status sph_time_kernel(sph_handle s, int stage, int reps, float* microsecond
                          s->status);
         }
     };
-    if (stage == ST_FORCE) {  // the masks of the current tuning
-        StepConfig c = s->cfg;
-        if (lists)
-            launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, c, false, true, st);
-        else
-            launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, c, st);
-    }
+    if (stage == ST_FORCE && !lists)  // the masks of the current tuning
+        launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, s->cfg, st);
     launch();  // warm
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    SPH_CUDA(cudaEventCreate(&e0));
-    cudaError_t e = cudaEventCreate(&e1);
+    cudaError_t e = cudaEventCreate(&e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
     if (e == cudaSuccess) {
         for (int r = 0; r < reps; r++) launch();
@@ -1654,8 +1676,15 @@ sph_status sph_time_kernel(sph_handle s, int stage, int reps, float* microsecond
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
+    if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
+    if (lists) {
+        for (Kept& k : kept)
+            if (e == cudaSuccess) e = cudaMemcpyAsync(k.at, k.copy, k.bytes, cudaMemcpyDeviceToDevice, st);
+        const cudaError_t w = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = w;
+        forget();
+    }
     SPH_CUDA(e);
     *microseconds = 1e3f * ms / (float)reps;
     return latched_status(s);

@@ -176,11 +176,12 @@ void enqueue_learned(sph_sim* s, Corrector* C) {
         launch_cell_scan(g.numCells, s->sb, s->status, st, &s->vl);
         launch_scatter(n, s->sb, st, s->status, &s->vl);
         launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, &s->vl, s->status);
-        launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, cfg, true, true, st);
+        launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), cfg, true,
+                             true, st);
         // the sorted copies are now this step's own: a reuse the audit granted is used up
         cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
         launch_force_learned(n, s->posS, s->velS, s->rho4S, s->sb.workIds, rows_of(s), g, ph, s->map,
-                             s->O.boxCollision, nullptr, nullptr, s->pos, s->vel, s->accS, cfg, fo, mdev(C),
+                             s->O.boxCollision, s->rowStart, s->rowMask, s->pos, s->vel, s->accS, cfg, fo, mdev(C),
                              s->status, st, &s->vl);
         s->lastStepLists = true;
         return;
@@ -204,7 +205,7 @@ void enqueue_audit(sph_sim* s, Corrector* C) {
     // same neighbours; it writes every particle's new state.
     if (s->vlOn)
         launch_force_lists(s->n, s->posS, s->velS, s->rho4S, s->sb.workIds, make_phys(s->P, s->O), s->map,
-                           s->O.boxCollision, s->vl, s->pos, s->vel, s->accS, s->cfg, q);
+                           s->O.boxCollision, s->vl, masks_of(s), s->pos, s->vel, s->accS, s->cfg, q);
     else
         launch_force(s->n, s->posS, s->velS, s->rho4S, s->sb.workIds, rows_of(s), grid_of(s),
                      make_phys(s->P, s->O), s->map, s->O.boxCollision, s->rowStart, s->rowMask, s->pos, s->vel,

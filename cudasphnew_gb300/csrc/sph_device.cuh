@@ -238,6 +238,12 @@ __device__ __forceinline__ bool row_window(float4 xi, int y, int z, float R, flo
     return e > s;
 }
 
+// Window w of a particle whose list holds windows (VL_WINDOWS).
+__device__ __forceinline__ int2 list_window(const NeighbourLists& L, int n, int i, int w) {
+    const int4 q = L.list[(size_t)(w >> 1) * n + i];
+    return (w & 1) ? make_int2(q.z, q.w) : make_int2(q.x, q.y);
+}
+
 // The cell range [lo, hi] of axis `a` that [p - r, p + r] touches, clamped to the grid.
 __device__ __forceinline__ void cell_span(float p, float r, const GridDev& g, int a, int& lo, int& hi) {
     const float inv = 1.0f / g.spacing;

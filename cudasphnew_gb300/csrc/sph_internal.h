@@ -126,17 +126,20 @@ struct RowTables {
 };
 
 // Reused neighbour lists (sph_options.neighbourSkin).  When the lists are
-// built, every particle records the stencil rows of the reference grid that
-// its skin sphere (radius R = (1 + skin) h) reaches: per row a window start
-// in the working order and a 64-bit mask of the candidates within R.  Later
-// steps keep that working order (the state is gathered into it) and visit
-// only those candidates, until some particle has moved farther than 0.45 skin
-// h from where it was at the build.  Slots 0-8 hold the reference's own 3 x 3
-// rows in its order (an empty row: start 0, no bits), so a build step sums
-// exactly what the per-step search sums; the further rows the skin reaches
-// follow from slot 9.  A window whose candidates within R span more than 64
-// places is kept unmasked: bit 31 of `start` set and the window end in the
-// low word of its masks.
+// built, every particle records the sorted slots of the particles within its
+// skin sphere (radius R = (1 + skin) h), itself among them, row by row of the
+// stencil in the working order, four to a group (the last group filled up
+// with slot n, a record far from everything that the sorted copies keep there).
+// Later steps keep that working order (the state is gathered into it) and
+// visit only those candidates, until some particle has moved farther than
+// 0.45 skin h from where it was at the build.  A particle with more than
+// VL_CAP candidates records its rows' windows [start, end) instead, two to a
+// group, and tests every particle in them.
+//
+// Why flat lists: with one bit mask per stencil row the lanes of a warp wait
+// at every row for the one with most neighbours there (21 of 32 lanes active,
+// ~55 gathers for 30 neighbours, each waited for alone); over a flat list
+// they wait once, and a group's four gathers are in flight together.
 // Batched handles keep one set of flags per scene (field-major: field f of
 // scene k at flags[f * numScenes + k]); each scene decides its builds from
 // its own particles' displacement and its own h, so a scene in a batch
@@ -144,15 +147,24 @@ struct RowTables {
 // from slotScene (the .w lane of the sorted position, which carries the
 // scene in the batch's other kernels, holds p/rho^2 once a list density
 // kernel has run).
-constexpr int VL_SLOTS = 16;  // rows within R <= 1.4 gridSpacing: at most 4 x 4
-constexpr int VL_INNER = 9;
+constexpr int VL_GROUPS = 24;            // list groups of a particle
+constexpr int VL_CAP = 4 * VL_GROUPS;    // candidates they hold (~40 at the default skin in a fluid at rest)
+constexpr int VL_ROWS = 16;              // rows within R <= 1.4 gridSpacing: at most 4 x 4
+constexpr unsigned int VL_WINDOWS = 0x80u;  // `groups` of a particle that records windows: this plus their number
+static_assert(VL_ROWS <= 2 * VL_GROUPS && VL_GROUPS < (int)VL_WINDOWS, "windows fit the groups");
 enum : int {
     VL_BUILD = 0,      // a build is requested (state written, another kind of step ran)
-    VL_BUILD_NOW = 1,  // this step builds the lists (decided at the start of the step)
+    VL_BUILD_NOW = 1,  // this step's kind, a VL_REUSES ... (decided at the start of the step)
     VL_DISP = 2,       // largest squared displacement since the build (float bits)
     VL_COUNT = 3,      // builds so far
     VL_FLAGS = 4,
 };
+// A step reuses the lists, builds them, or searches without building: when a
+// step has moved some particle past the rebuild distance by itself, lists
+// built for it were never used, and the steps that follow search as a handle
+// without lists does (recording windows of radius h) until one stays within
+// the distance again.
+enum : unsigned int { VL_REUSES = 0, VL_BUILDS = 1, VL_SEARCHES = 2 };
 // Two words after the per-scene flags: whether this step sorts (some scene
 // builds; a step that builds nothing keeps the working order and skips the
 // hash, scan and scatter), and whether the cell tables on the device are
@@ -160,12 +172,8 @@ enum : int {
 // from that step's sorted copies).
 enum : int { VL_SORT = 0, VL_STALE = 1, VL_GLOBAL = 2 };
 struct NeighbourLists {
-    int* start;            // [VL_SLOTS][n] window start (bit 31: unmasked window)
-    uint2* skin;           // [VL_SLOTS][n] candidates within R (bit k: start + k; .x bits 0-31), or
-                           //               .x = the window end
-    uint2* exact;          // [VL_SLOTS][n] this step's neighbours (0 < r <= h) over the same window, or
-                           //               .x = the window end
-    unsigned char* rows;   // [n] slots in use (9 + the further rows)
+    int4* list;            // [VL_GROUPS][n] candidates within R, or two windows [start, end) a group
+    unsigned char* groups; // [n] groups in use, or VL_WINDOWS + windows in use
     float4* posB;          // [n] positions at the build, working order
     unsigned int* flags;   // [VL_FLAGS][numScenes], then [VL_GLOBAL]
     float radius, radius2; // R and R^2 (single-scene handles; a batch's kernels take each scene's h)
@@ -174,6 +182,13 @@ struct NeighbourLists {
     int numScenes;         // 1, or the batch's scene count
     int* slotScene;        // batched handles: [n] the scene of each sorted slot (a scene's particles
                            // always fill the same slot range: its cells follow the previous scene's)
+};
+
+// What the density stage records for the force stage of the per-step search,
+// and of a step that builds the lists.
+struct RowMasks {
+    int* start;          // [9][n] window start, bit 31 set when the row was not masked
+    unsigned int* mask;  // [9][n] neighbour bits relative to start, or the window end
 };
 
 // Launch configuration of the step (chosen per handle; see the autotuner).
@@ -253,24 +268,28 @@ void launch_rank_gather(int n, SortBuffers sb, const float4* pos, const float4* 
                         float4* posS, float4* velS, cudaStream_t s, const NeighbourLists* lists = nullptr,
                         unsigned int* status = nullptr);
 // Density stage over reused neighbour lists: the build form (the reference's
-// rows and the skin rows, recording the lists) and the list form; each
-// returns at once unless the step is of its kind.
+// rows and the skin rows, recording the lists, and in M this step's
+// neighbours by row) and the list form; each returns at once unless the step
+// is of its kind.
 // Besides rho4S, each particle's p/rho^2 and 1/rho go to the fourth lanes of
 // its sorted position and velocity, where the list force stage reads them.
 void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                          float4* rho4S, const NeighbourLists& L, const StepConfig& cfg, bool build, bool reuse,
-                          cudaStream_t s);
+                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg, bool build,
+                          bool reuse, cudaStream_t s);
 // After a write of the positions: the largest distance from the build
 // positions, measured afresh (the lists stay if it is within the limit).
 // (Batched handles: each particle's scene from the .w lane of its position.)
 void launch_list_displacement(int n, const float4* pos, const int* workIds, const NeighbourLists& L,
                               cudaStream_t s);
-// Force stage over the lists' neighbour masks; also records the largest
-// displacement since the build.  With `scenes` (batched handles) each
+// Force stage over the lists, or over M's rows in a step that builds them;
+// also records the largest displacement since the build.  With `scenes` (batched handles) each
 // particle's constants and maps come from its scene's record.
 void launch_force_lists(int n, const float4* posS, const float4* velS, const float4* rho4S, const int* workIds,
-                        PhysDev ph, MapDev map, int collide, const NeighbourLists& L, float4* pos, float4* vel,
-                        float4* accS, const StepConfig& cfg, cudaStream_t s, const SceneDev* scenes = nullptr);
+                        PhysDev ph, MapDev map, int collide, const NeighbourLists& L, RowMasks M, float4* pos,
+                        float4* vel, float4* accS, const StepConfig& cfg, cudaStream_t s,
+                        const SceneDev* scenes = nullptr);
+// The far record that a list's unused entries name: posS[n], velS[n].
+void launch_list_far_record(int n, float4* posS, float4* velS, cudaStream_t s);
 void launch_density(int n, const float4* posS, RowTables T, GridDev g, PhysDev ph, MapDev map,
                     float4* rho4S, int* rowStart, unsigned int* rowMask, const StepConfig& cfg,
                     cudaStream_t s);

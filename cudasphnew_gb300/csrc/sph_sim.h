@@ -144,6 +144,7 @@ struct sph_sim {
 namespace sph {
 
 RowTables rows_of(const sph_sim* s);
+RowMasks masks_of(const sph_sim* s);
 GridDev make_grid(const SimulationParameters& P, bool sub);
 PhysDev make_phys(const SimulationParameters& P, const sph_options& O);
 PhysDev make_sub_phys(const SimulationParameters& P, const sph_options& O);

@@ -172,7 +172,8 @@ static int stride_blocks(int n) {
 // Reused neighbour lists: whether each scene builds them in this step (on
 // request, or when one of its particles has moved farther than the skin
 // allows since the last build, or the displacement is not finite; thread k
-// decides scene k), whether the step sorts (some scene builds) and whether
+// decides scene k; VL_SEARCHES in place of a build that the last step's own
+// displacement would have outrun), whether the step sorts (some scene builds) and whether
 // it leaves the cell tables stale (it does not sort).  One block.
 __global__ void k_list_decide(NeighbourLists L, const SceneDev* __restrict__ scenes) {
     __shared__ int anyBuild;
@@ -187,12 +188,17 @@ __global__ void k_list_decide(NeighbourLists L, const SceneDev* __restrict__ sce
             lim2 = lim * lim;
         }
         const float d2 = __uint_as_float(f[VL_DISP * S + k]);
-        const bool build = f[VL_BUILD * S + k] != 0u || !(d2 <= lim2);
-        f[VL_BUILD_NOW * S + k] = build ? 1u : 0u;
+        const bool asked = f[VL_BUILD * S + k] != 0u, past = !(d2 <= lim2);
+        const unsigned int last = f[VL_BUILD_NOW * S + k];
+        const unsigned int kind = asked                ? VL_BUILDS
+                                  : past               ? (last == VL_REUSES ? VL_BUILDS : VL_SEARCHES)
+                                  : last == VL_SEARCHES ? VL_BUILDS
+                                                        : VL_REUSES;
+        f[VL_BUILD_NOW * S + k] = kind;
         f[VL_BUILD * S + k] = 0u;
-        if (build) {
+        if (kind != VL_REUSES) {
             f[VL_DISP * S + k] = 0u;
-            f[VL_COUNT * S + k] += 1u;
+            if (kind == VL_BUILDS) f[VL_COUNT * S + k] += 1u;
             anyBuild = 1;
         }
     }

@@ -31,11 +31,6 @@ namespace sph {
 // Branch-free poly6 accumulation: max(h^2 - r^2, 0)^3.  Writes
 // (rho, p, p/rho^2, 1/rho) for the force stage.
 // ---------------------------------------------------------------------------
-struct RowMasks {
-    int* start;          // [9][n] window start, bit 31 set when the row was not masked
-    unsigned int* mask;  // [9][n] neighbour bits relative to start, or the window end
-};
-
 // With REL the positions are cell-relative: every neighbour is moved into
 // particle i's cell frame before its distance is taken.
 // Occupancy: 40 registers (six 256-thread blocks per SM) cost no spills
@@ -106,14 +101,17 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
 // Density over reused neighbour lists (sph_options.neighbourSkin).
 //
 // Build form (steps that build the lists): the reference's 3 x 3 stencil
-// rows first, in its order, into slots 0-8, then the further rows the skin
-// sphere of radius R reaches; each row's window at R is walked in the working
-// order and the density terms are summed as in k_density (candidates beyond
-// h add exactly nothing, so the reference's rows give the same row sums).
-// Each row is recorded with two 64-bit masks over its candidates, starting at
-// its first candidate within R: the candidates within R (the lists) and the
-// neighbours within h (this step's force stage).  A row whose candidates
-// within R span more than 64 places is kept unmasked.
+// rows first, in its order, then the further rows the skin sphere of radius R
+// reaches; each row's window at R is walked in the working order.  The
+// reference's rows give the density terms, summed as in k_density (candidates
+// beyond h add exactly nothing, so the row sums are the same), and this
+// step's neighbours by row for the force stage; every row gives its
+// candidates within R to the particle's list.  A step that searches without
+// building (VL_SEARCHES) takes windows at h and records those.
+//
+// A row is tested 32 candidates at a time into two bit masks (within R,
+// within h; one multiply-add each), and only the set bits are appended: the
+// append costs ten times the test and a third of the candidates pass.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ bool within_r2(float r2, float R2) {  // r2 >= 0 or NaN
     return __float_as_uint(r2) <= __float_as_uint(R2);
@@ -124,83 +122,108 @@ __device__ __forceinline__ bool within_r2(float r2, float R2) {  // r2 >= 0 or N
 template <bool KAHAN, bool BATCH>
 __device__ __forceinline__ void density_build_one(int i, int n, float4* posS, float4* velS, const RowTables& T,
                                                   const GridDev& g_, const PhysDev& ph_, const MapDev& map_,
-                                                  float4* __restrict__ rho4S, const NeighbourLists& L) {
+                                                  float4* __restrict__ rho4S, const NeighbourLists& L,
+                                                  const RowMasks& M) {
     const int scene = BATCH ? L.slotScene[i] : 0;
-    if (!L.flags[VL_BUILD_NOW * L.numScenes + scene]) return;
+    const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
+    if (kind == VL_REUSES) return;
+    const bool lists = kind == VL_BUILDS;
     const float4 xi = posS[i];
     const SceneDev* S = BATCH ? T.scenes + scene : nullptr;
     const GridDev& g = BATCH ? S->g : g_;
     const PhysDev& ph = BATCH ? S->ph : ph_;
     const MapDev& map = BATCH ? S->map : map_;
     const Stencil st = stencil(xi, ph.h, g);
-    const float R = BATCH ? (1.0f + L.skinFrac) * ph.h : L.radius;
+    const float R = !lists ? ph.h : BATCH ? (1.0f + L.skinFrac) * ph.h : L.radius;
     const float h2 = ph.h2, R2 = BATCH ? R * R : L.radius2, eps = 1e-3f * ph.h;
     float sum = 0.f, comp = 0.f;
-    int extra = VL_INNER;  // next slot of a further row
-    // `slot` >= 0: a fixed slot, written even when the row is empty
+    int count = 0;
+    int4 group = make_int4(n, n, n, n);
+    auto append = [&](int t) {
+        group = make_int4(group.y, group.z, group.w, t);
+        count++;
+        if ((count & 3) == 0 && count <= VL_CAP) L.list[(size_t)((count >> 2) - 1) * n + i] = group;
+    };
+    // row (y, z); slot >= 0: one of the reference's rows, recorded even when empty
     auto visit = [&](int y, int z, int slot) {
         int s0 = 0, e0 = 0;
-        const bool any = y >= 0 && row_window(xi, y, z, R, eps, g, T, s0, e0);
+        if (y >= 0) row_window(xi, y, z, R, eps, g, T, s0, e0);
         float rs = 0.f;
-        unsigned long long ms = 0ull, me = 0ull;  // bit t - first, for the first 64
         int first = -1, last = -1;
-        if (any) {
-            for (int t = s0; t < e0; t++) {
-                const float4 xj = __ldg(posS + t);
-                const float r2 = dist2(xi, xj);
+        unsigned int m = 0u;  // neighbours within h, bit t - first
+        for (int base = s0; base < e0; base += 32) {
+            const int c = min(32, e0 - base);
+            unsigned int mR = 0u, mh = 0u;  // first candidate in the highest bit used, turned around below
+#pragma unroll 2
+            for (int t = base; t < base + c; t++) {
+                const float r2 = dist2(xi, __ldg(posS + t));
                 const float w = fmaxf(h2 - r2, 0.f);
                 rs = fmaf(w * w, w, rs);
-                if (within_r2(r2, R2)) {
-                    if (first < 0) first = t;
-                    last = t;
-                    const int k = t - first;
-                    if (k < 64) {
-                        ms |= 1ull << k;
-                        if (neighbour_r2(r2, h2)) me |= 1ull << k;
-                    }
+                mR = mR * 2u + (within_r2(r2, R2) ? 1u : 0u);
+                mh = mh * 2u + (neighbour_r2(r2, h2) ? 1u : 0u);
+            }
+            mR = lists ? __brev(mR) >> (32 - c) : 0u;
+            mh = __brev(mh) >> (32 - c);
+            if (mh) {
+                if (first < 0) {
+                    const int k = __ffs(mh) - 1;
+                    first = base + k;
+                    m = mh >> k;
+                } else if (base - first < 32) {
+                    m |= mh << (base - first);
                 }
+                last = base + 31 - __clz(mh);
+            }
+            while (mR) {
+                const int k = __ffs(mR) - 1;
+                mR &= mR - 1u;
+                append(base + k);
             }
         }
+        if (slot < 0) return;
         if (KAHAN) {
             if (rs > 0.f) kahan_add(sum, comp, rs);
         } else {
             sum += rs;
         }
-        if (slot < 0) {
-            if (first < 0 || extra >= VL_SLOTS) return;  // nothing within R to record
-            slot = extra++;
-        }
+        const bool fits = last - first < 32;
         const size_t at = (size_t)slot * n + i;
-        if (first < 0) {
-            L.start[at] = 0;
-            L.skin[at] = make_uint2(0u, 0u);
-            L.exact[at] = make_uint2(0u, 0u);
-        } else if (last - first < 64) {
-            L.start[at] = first;
-            L.skin[at] = make_uint2((unsigned int)ms, (unsigned int)(ms >> 32));
-            L.exact[at] = make_uint2((unsigned int)me, (unsigned int)(me >> 32));
-        } else {
-            L.start[at] = first | (int)0x80000000;
-            L.skin[at] = make_uint2((unsigned int)(last + 1), 0u);
-            L.exact[at] = make_uint2((unsigned int)(last + 1), 0u);
-        }
+        M.start[at] = first < 0 ? 0 : fits ? first : (first | (int)0x80000000);
+        M.mask[at] = fits ? m : (unsigned int)(last + 1);
     };
-    // the reference's rows (k_density's order) into their slots, then the rest within R
+    // the reference's rows (k_density's order), then the rest within R
     const int y1 = min(st.y1, st.y0 + 2), z1 = min(st.z1, st.z0 + 2);
-#pragma unroll 1
-    for (int r = 0; r < VL_INNER; r++) {
-        const int z = st.z0 + r / 3, y = st.y0 + r % 3;
-        visit(z <= z1 && y <= y1 ? y : -1, z, r);
-    }
     int ya, yb, za, zb;
     cell_span(xi.y, R + eps, g, 1, ya, yb);
     cell_span(xi.z, R + eps, g, 2, za, zb);
+    auto rows = [&](auto&& row) {
 #pragma unroll 1
-    for (int z = za; z <= zb; z++)
+        for (int r = 0; r < 9; r++) {
+            const int z = st.z0 + r / 3, y = st.y0 + r % 3;
+            row(z <= z1 && y <= y1 ? y : -1, z, r);
+        }
+        if (!lists) return;
 #pragma unroll 1
-        for (int y = ya; y <= yb; y++)
-            if (z < st.z0 || z > z1 || y < st.y0 || y > y1) visit(y, z, -1);
-    L.rows[i] = (unsigned char)extra;
+        for (int z = za; z <= zb; z++)
+#pragma unroll 1
+            for (int y = ya; y <= yb; y++)
+                if (z < st.z0 || z > z1 || y < st.y0 || y > y1) row(y, z, -1);
+    };
+    rows(visit);
+    if (lists && count <= VL_CAP) {
+        L.groups[i] = (unsigned char)((count + 3) >> 2);
+        while (count & 3) append(n);
+    } else {
+        // too many for the list, or no list to build: the rows' windows
+        int w = 0;
+        rows([&](int y, int z, int) {
+            int s0 = 0, e0 = 0;
+            if (y < 0 || w >= VL_ROWS || !row_window(xi, y, z, R, eps, g, T, s0, e0)) return;
+            reinterpret_cast<int2*>(L.list + (size_t)(w >> 1) * n + i)[w & 1] = make_int2(s0, e0);
+            w++;
+        });
+        L.groups[i] = (unsigned char)(VL_WINDOWS + w);
+    }
     L.posB[i] = xi;
     float rho = (KAHAN ? __fsub_rn(sum, comp) : sum) * ph.poly6m;
     if (map.present) {
@@ -222,18 +245,18 @@ __device__ __forceinline__ void density_build_one(int i, int n, float4* posS, fl
 template <bool KAHAN, bool BATCH>
 __global__ void __launch_bounds__(256, 4)
 k_density_build(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                float4* __restrict__ rho4S, NeighbourLists L) {
+                float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
     if (!BATCH && !L.flags[VL_BUILD_NOW]) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        density_build_one<KAHAN, BATCH>(i, n, posS, velS, T, g, ph, map, rho4S, L);
+        density_build_one<KAHAN, BATCH>(i, n, posS, velS, T, g, ph, map, rho4S, L, M);
 }
 
-// List form: each recorded row's candidates within R, in the recorded order;
-// the row's neighbours within h of this step are recorded for the force
-// stage over the same window (empty and unmasked rows keep what the build
-// wrote).  The next row's entries are loaded before the current row is walked.
+// List form: the candidates within R, four at a time; each group's terms are
+// summed in plain FP32 (as a row's few terms are) and the group sums are
+// added with compensation.  The next group's slots are loaded before the
+// current group's positions are used.
 template <bool KAHAN, bool BATCH>
-__global__ void __launch_bounds__(256, 8)
+__global__ void __launch_bounds__(256, 6)
 k_density_lists(int n, float4* posS, float4* velS, PhysDev ph_, MapDev map_, float4* __restrict__ rho4S,
                 NeighbourLists L, const SceneDev* __restrict__ scenes) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -244,50 +267,35 @@ k_density_lists(int n, float4* posS, float4* velS, PhysDev ph_, MapDev map_, flo
     const PhysDev& ph = BATCH ? scenes[scene].ph : ph_;
     const MapDev& map = BATCH ? scenes[scene].map : map_;
     const float h2 = ph.h2;
-    const int rows = L.rows[i];
+    const unsigned int groups = L.groups[i];
     float sum = 0.f, comp = 0.f;
-    int svN = __ldg(L.start + i);
-    uint2 mN = __ldg(L.skin + i);
+    auto total = [&](float rs) {
+        if (KAHAN) kahan_add(sum, comp, rs);
+        else sum += rs;
+    };
+    if (!(groups & VL_WINDOWS)) {
+        const int4* lp = L.list + i;
+        int4 c = groups ? __ldg(lp) : make_int4(0, 0, 0, 0);
 #pragma unroll 1
-    for (int r = 0; r < rows; r++) {
-        const int sv = svN;
-        const uint2 m = mN;
-        if (r + 1 < rows) {
-            svN = __ldg(L.start + (size_t)(r + 1) * n + i);
-            mN = __ldg(L.skin + (size_t)(r + 1) * n + i);
+        for (unsigned int k = 0; k < groups; k++) {
+            const float4 x0 = __ldg(posS + c.x), x1 = __ldg(posS + c.y), x2 = __ldg(posS + c.z),
+                         x3 = __ldg(posS + c.w);
+            lp += n;
+            if (k + 1 < groups) c = __ldg(lp);
+            const float w0 = fmaxf(h2 - dist2(xi, x0), 0.f), w1 = fmaxf(h2 - dist2(xi, x1), 0.f);
+            const float w2 = fmaxf(h2 - dist2(xi, x2), 0.f), w3 = fmaxf(h2 - dist2(xi, x3), 0.f);
+            total(fmaf(w3 * w3, w3, fmaf(w2 * w2, w2, fmaf(w1 * w1, w1, w0 * w0 * w0))));
         }
-        float rs = 0.f;
-        if (sv < 0) {
-            for (int t = sv & 0x7fffffff; t < (int)m.x; t++) {
-                const float w = fmaxf(h2 - dist2(xi, __ldg(posS + t)), 0.f);
-                rs = fmaf(w * w, w, rs);
+    } else {
+#pragma unroll 1
+        for (unsigned int w = 0; w < groups - VL_WINDOWS; w++) {
+            const int2 se = list_window(L, n, i, (int)w);
+            float rs = 0.f;
+            for (int t = se.x; t < se.y; t++) {
+                const float d = fmaxf(h2 - dist2(xi, __ldg(posS + t)), 0.f);
+                rs = fmaf(d * d, d, rs);
             }
-        } else if (m.x | m.y) {
-            unsigned int e0 = 0u, e1 = 0u;
-            unsigned int b = m.x;
-            while (b) {
-                const int k = __ffs(b) - 1;
-                b &= b - 1u;
-                const float r2 = dist2(xi, __ldg(posS + sv + k));
-                const float w = fmaxf(h2 - r2, 0.f);
-                rs = fmaf(w * w, w, rs);
-                if (neighbour_r2(r2, h2)) e0 |= 1u << k;
-            }
-            b = m.y;
-            while (b) {
-                const int k = __ffs(b) - 1;
-                b &= b - 1u;
-                const float r2 = dist2(xi, __ldg(posS + sv + 32 + k));
-                const float w = fmaxf(h2 - r2, 0.f);
-                rs = fmaf(w * w, w, rs);
-                if (neighbour_r2(r2, h2)) e1 |= 1u << k;
-            }
-            L.exact[(size_t)r * n + i] = make_uint2(e0, e1);
-        }
-        if (KAHAN) {
-            if (rs > 0.f) kahan_add(sum, comp, rs);
-        } else {
-            sum += rs;
+            total(rs);
         }
     }
     float rho = (KAHAN ? __fsub_rn(sum, comp) : sum) * ph.poly6m;
@@ -303,6 +311,17 @@ k_density_lists(int n, float4* posS, float4* velS, PhysDev ph_, MapDev map_, flo
     // velocity rides in their unused fourth lanes: two loads per pair, not three
     posS[i].w = p * inv * inv;
     velS[i].w = inv;
+}
+
+// The far record: r^2 of any particle to it is ~3e36, beyond every support
+// and finite.
+__global__ void k_list_far_record(int n, float4* posS, float4* velS) {
+    posS[n] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+    velS[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+void launch_list_far_record(int n, float4* posS, float4* velS, cudaStream_t s) {
+    k_list_far_record<<<1, 1, 0, s>>>(n, posS, velS);
 }
 
 // ---------------------------------------------------------------------------
@@ -403,6 +422,9 @@ struct ForceTotals {
     float cg[3] = {0.f, 0.f, 0.f}, cl = 0.f;
     __device__ __forceinline__ void add(const RowSums<TENSION>& r) {
         if (r.hits == 0) return;
+        add_all(r);
+    }
+    __device__ __forceinline__ void add_all(const RowSums<TENSION>& r) {
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             if (KAHAN) {
@@ -755,19 +777,81 @@ __global__ void __launch_bounds__(256, FEAT ? 3 : (BATCH || TENSION || REL || FO
 }
 
 // ---------------------------------------------------------------------------
-// Force stage over reused neighbour lists: the pretested form over the rows
-// the lists recorded (the density stage wrote this step's neighbour masks
-// over them), then wall terms, integration, collision and write-back as
-// k_force.  The next row's entries are loaded before the current row is
-// walked.  It also records, for the decision at the next step, the largest
+// Force stage over reused neighbour lists, then wall terms, integration,
+// collision and write-back as k_force.  A reusing step walks the lists: four
+// candidates at a time, their eight records in flight together, those beyond
+// h left out of the sums; a group's terms are summed in plain FP32 and the
+// group sums added with compensation, as a row's are.  A building step takes
+// the rows that the density stage recorded, so it adds exactly what k_force
+// adds.  It also records, for the decision at the next step, the largest
 // squared distance of a particle from where it was when the lists were built.
-// Occupancy: at most 56 registers, so nine 128-thread blocks fit on an SM
-// (36 warps; at 64 registers eight): the single-scene forms spill 4-16
-// bytes, the batched ones up to 88, and both run 1-2 % faster per step than
-// at 64 registers without spills.  At 48 registers (ten blocks) the spills
-// cost more than the warps gain.  A register cap, not a launch bound, so any
-// block size the autotuner tries stays launchable.
 // ---------------------------------------------------------------------------
+// The neighbours of a list step's particle: `pair` for each candidate (with
+// `tested` when it is known to lie within h), `row` with the sums of each
+// row's, window's or (group true) list group's pairs.
+template <bool TENSION, class PAIR, class ROW>
+__device__ __forceinline__ void list_rows(int i, int n, int scene, const NeighbourLists& L, const RowMasks& M,
+                                          const float4* __restrict__ posS, const float4* __restrict__ velS,
+                                          PAIR&& pair, ROW&& row) {
+    if (L.flags[VL_BUILD_NOW * L.numScenes + scene]) {
+        int svN = __ldg(M.start + i);
+        unsigned int mN = __ldg(M.mask + i);
+#pragma unroll 1
+        for (int r = 0; r < 9; r++) {
+            const int sv = svN;
+            unsigned int m = mN;
+            if (r + 1 < 9) {
+                svN = __ldg(M.start + (size_t)(r + 1) * n + i);
+                mN = __ldg(M.mask + (size_t)(r + 1) * n + i);
+            }
+            RowSums<TENSION> R;
+            R.clear();
+            if (sv < 0) {
+                for (int t = sv & 0x7fffffff; t < (int)m; t++) pair(R, __ldg(posS + t), __ldg(velS + t), false);
+            } else {
+                while (m) {
+                    const int t = sv + __ffs(m) - 1;
+                    m &= m - 1u;
+                    pair(R, __ldg(posS + t), __ldg(velS + t), true);
+                }
+            }
+            row(R, false);
+        }
+        return;
+    }
+    const unsigned int groups = L.groups[i];
+    if (groups & VL_WINDOWS) {
+#pragma unroll 1
+        for (unsigned int w = 0; w < groups - VL_WINDOWS; w++) {
+            const int2 se = list_window(L, n, i, (int)w);
+            RowSums<TENSION> R;
+            R.clear();
+            for (int t = se.x; t < se.y; t++) pair(R, __ldg(posS + t), __ldg(velS + t), false);
+            row(R, false);
+        }
+        return;
+    }
+    const int4* lp = L.list + i;
+    int4 c = groups ? __ldg(lp) : make_int4(0, 0, 0, 0);
+#pragma unroll 1
+    for (unsigned int k = 0; k < groups; k++) {
+        const float4 x0 = __ldg(posS + c.x), x1 = __ldg(posS + c.y), x2 = __ldg(posS + c.z), x3 = __ldg(posS + c.w);
+        const float4 v0 = __ldg(velS + c.x), v1 = __ldg(velS + c.y), v2 = __ldg(velS + c.z), v3 = __ldg(velS + c.w);
+        lp += n;
+        if (k + 1 < groups) c = __ldg(lp);
+        RowSums<TENSION> R;
+        R.clear();
+        pair(R, x0, v0, false);
+        pair(R, x1, v1, false);
+        pair(R, x2, v2, false);
+        pair(R, x3, v3, false);
+        row(R, true);
+    }
+}
+
+#ifndef FORCE_REGS
+#define FORCE_REGS 72
+#endif
 // Displacement since the build into the scene's flag: one atomic per warp (or
 // per scene a warp holds) that raises the recorded maximum.  Squared
 // distances are non-negative, so their bits order as the values do; the
@@ -784,10 +868,10 @@ __device__ __forceinline__ void record_displacement(const NeighbourLists& L, int
 }
 
 template <bool KAHAN, bool TENSION, bool BATCH>
-__global__ void __maxnreg__(56)
+__global__ void __maxnreg__(FORCE_REGS)
 k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__ velS,
               const float4* __restrict__ rho4S, const int* __restrict__ workIds, PhysDev ph_, MapDev map_,
-              int collideFlag, NeighbourLists L, float4* __restrict__ pos, float4* __restrict__ vel,
+              int collideFlag, NeighbourLists L, RowMasks M, float4* __restrict__ pos, float4* __restrict__ vel,
               float4* __restrict__ accS, const SceneDev* __restrict__ scenes) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float d2 = 0.f;
@@ -801,44 +885,19 @@ k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__
         const MapDev& map = BATCH ? scenes[scene].map : map_;
         const float h2 = ph.h2;
         ForceTotals<KAHAN, TENSION> A;
-        const int rows = L.rows[i];
-        int svN = __ldg(L.start + i);
-        uint2 mN = __ldg(L.exact + i);
-        // a neighbour's p/rho^2 and 1/rho ride in the fourth lanes of its
-        // sorted position and velocity (written by the density stage)
-        auto pairs = [&](RowSums<TENSION>& R, int base, unsigned int m) {
-            R.hits += __popc(m);
-            while (m) {
-                const int t = base + __ffs(m) - 1;
-                m &= m - 1u;
-                const float4 xj = __ldg(posS + t), vj = __ldg(velS + t);
-                R.template add<false>(ph, Pair(ph, xi, vi, xj, vj), ri.z, make_float4(0.f, 0.f, xj.w, vj.w));
-            }
-        };
-#pragma unroll 1
-        for (int r = 0; r < rows; r++) {
-            const int sv = svN;
-            const uint2 m = mN;
-            if (r + 1 < rows) {
-                svN = __ldg(L.start + (size_t)(r + 1) * n + i);
-                mN = __ldg(L.exact + (size_t)(r + 1) * n + i);
-            }
-            RowSums<TENSION> R;
-            R.clear();
-            if (sv < 0) {
-                for (int t = sv & 0x7fffffff; t < (int)m.x; t++) {
-                    const float4 xj = __ldg(posS + t);
-                    if (neighbour_r2(dist2(xi, xj), h2)) {
-                        const float4 vj = __ldg(velS + t);
-                        R.add(ph, Pair(ph, xi, vi, xj, vj), ri.z, make_float4(0.f, 0.f, xj.w, vj.w));
-                    }
-                }
-            } else {
-                pairs(R, sv, m.x);
-                pairs(R, sv + 32, m.y);
-            }
-            A.add(R);
-        }
+        // (a neighbour's p/rho^2 and 1/rho ride in the fourth lanes of its
+        // sorted position and velocity, written by the density stage)
+        list_rows<TENSION>(
+            i, n, scene, L, M, posS, velS,
+            [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
+                const Pair p(ph, xi, vi, xj, vj);
+                if (tested || neighbour_r2(p.r2, h2))
+                    R.add(ph, p, ri.z, make_float4(0.f, 0.f, xj.w, vj.w));
+            },
+            [&](const RowSums<TENSION>& R, bool group) {
+                if (group) A.add_all(R);
+                else A.add(R);
+            });
         float mapDist = 1e30f, mapN[3] = {0.f, 0.f, 0.f};
         float3 x, v;
         float acc[3];
@@ -1039,11 +1098,11 @@ static_assert(L_X % 1024 == 0 && L_BIAS % 16 == 0 && L_NORM % 16 == 0 && L_BAR %
 static_assert(L_BLOCKS_MAX * (L_SMEM + 1024) <= 227 * 1024 && L_BLOCKS_MAX * L_TMEM <= 512,
               "resident blocks per SM");
 
-// LISTS: the neighbours come from the reused lists' exact masks (as in
-// k_force_lists: the same pairs in the same order as the masks of the
-// per-step search at a building step, the neighbours' p/rho^2 and 1/rho from
-// the fourth lanes of their sorted position and velocity), and the kernel
-// records the largest squared distance of a corrected position from where
+// LISTS: the neighbours come from the reused lists, or in a building step
+// from the rows the density stage recorded (as in k_force_lists; the same
+// pairs in the same order as the per-step search there), their p/rho^2 and
+// 1/rho from the fourth lanes of their sorted position and velocity, and the
+// kernel records the largest squared distance of a corrected position from where
 // the particle was when the lists were built.
 template <bool KAHAN, bool TENSION, int BLOCKS, bool LISTS>
 __global__ void __launch_bounds__(L_THREADS, BLOCKS)
@@ -1085,42 +1144,21 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
             ForceTotals<KAHAN, TENSION> A;
             FeatSums fs;
             if (LISTS) {
-                const int rows = L.rows[i];
-#pragma unroll 1
-                for (int row = 0; row < rows; row++) {
-                    RowSums<TENSION> R;
-                    R.clear();
-                    const int sv = __ldg(L.start + (size_t)row * F.n + i);
-                    const uint2 mk = __ldg(L.exact + (size_t)row * F.n + i);
-                    if (sv < 0) {
-                        for (int tt = sv & 0x7fffffff; tt < (int)mk.x; tt++) {
-                            const float4 xj = __ldg(F.posS + tt);
-                            if (neighbour_r2(dist2(xi, xj), ph.h2)) {
-                                const float4 vj = __ldg(F.velS + tt), rj = make_float4(0.f, 0.f, xj.w, vj.w);
-                                const Pair p(ph, xi, vi, xj, vj);
-                                R.add(ph, p, ri.z, rj);
-                                fs.add(ph, p, rj);
-                            }
+                list_rows<TENSION>(
+                    i, F.n, 0, L, F.M, F.posS, F.velS,
+                    [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
+                        const Pair p(ph, xi, vi, xj, vj);
+                        if (tested || neighbour_r2(p.r2, ph.h2)) {
+                            const float4 rj = make_float4(0.f, 0.f, xj.w, vj.w);
+                            R.add(ph, p, ri.z, rj);
+                            fs.add(ph, p, rj);
                         }
-                    } else {
-                        R.hits += __popc(mk.x) + __popc(mk.y);
-#pragma unroll
-                        for (int w = 0; w < 2; w++) {
-                            unsigned int b = w ? mk.y : mk.x;
-                            while (b) {
-                                const int tt = sv + 32 * w + __ffs(b) - 1;
-                                b &= b - 1u;
-                                const float4 xj = __ldg(F.posS + tt), vj = __ldg(F.velS + tt);
-                                const float4 rj = make_float4(0.f, 0.f, xj.w, vj.w);
-                                const Pair p(ph, xi, vi, xj, vj);
-                                R.template add<false>(ph, p, ri.z, rj);
-                                fs.add(ph, p, rj);
-                            }
-                        }
-                    }
-                    A.add(R);
-                    fs.cnt += R.hits;
-                }
+                    },
+                    [&](const RowSums<TENSION>& R, bool group) {
+                        if (group) A.add_all(R);
+                        else A.add(R);
+                        fs.cnt += R.hits;
+                    });
             }
 #pragma unroll
             for (int row = 0; row < (LISTS ? 0 : 9); row++) {
@@ -1397,13 +1435,13 @@ void launch_list_displacement(int n, const float4* pos, const int* workIds, cons
 }
 
 void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                          float4* rho4S, const NeighbourLists& L, const StepConfig& cfg, bool build, bool reuse,
-                          cudaStream_t s) {
+                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg, bool build,
+                          bool reuse, cudaStream_t s) {
     if (n <= 0) return;
     const int bs = cfg.densityBlock > 0 ? cfg.densityBlock : 128;
     const int grid = (n + bs - 1) / bs;
     const bool batch = T.scenes != nullptr;
-#define SPH_DENSITY_BUILD(K, B) k_density_build<K, B><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L)
+#define SPH_DENSITY_BUILD(K, B) k_density_build<K, B><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L, M)
 #define SPH_DENSITY_LISTS(K, B) \
     k_density_lists<K, B><<<grid, bs, 0, s>>>(n, posS, velS, ph, map, rho4S, L, T.scenes)
     if (build) {
@@ -1429,8 +1467,8 @@ void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDe
 }
 
 void launch_force_lists(int n, const float4* posS, const float4* velS, const float4* rho4S, const int* workIds,
-                        PhysDev ph, MapDev map, int collide, const NeighbourLists& L, float4* pos, float4* vel,
-                        float4* accS, const StepConfig& cfg, cudaStream_t s, const SceneDev* scenes) {
+                        PhysDev ph, MapDev map, int collide, const NeighbourLists& L, RowMasks M, float4* pos,
+                        float4* vel, float4* accS, const StepConfig& cfg, cudaStream_t s, const SceneDev* scenes) {
     if (n <= 0) return;
     const int bs = cfg.forceBlock > 0 ? cfg.forceBlock : 128;
     const int grid = (n + bs - 1) / bs;
@@ -1438,7 +1476,7 @@ void launch_force_lists(int n, const float4* posS, const float4* velS, const flo
     // whether the colour field is computed at all)
     const bool tension = ph.tension != 0.0f;
 #define SPH_FORCE_LISTS(K, T, B)                                                                             \
-    k_force_lists<K, T, B><<<grid, bs, 0, s>>>(n, posS, velS, rho4S, workIds, ph, map, collide, L, pos, vel, \
+    k_force_lists<K, T, B><<<grid, bs, 0, s>>>(n, posS, velS, rho4S, workIds, ph, map, collide, L, M, pos, vel, \
                                                accS, scenes)
 #define SPH_FORCE_LISTS_B(K, T)           \
     do {                                  \

@@ -58,23 +58,28 @@ __global__ void k_surface_lists(int n, const float4* __restrict__ posS, const in
     const float h2 = h * h;
     double sx = 0.0, sy = 0.0, sz = 0.0;
     int cnt = 0;
-    const int rows = L.rows[u];
-    for (int r = 0; r < rows; r++) {
-        const size_t at = (size_t)r * n + u;
-        const int sv = L.start[at];
-        const uint2 m2 = L.skin[at];
-        const unsigned long long m = (unsigned long long)m2.x | ((unsigned long long)m2.y << 32);
-        const int t0 = sv & 0x7fffffff;
-        const int t1 = sv < 0 ? (int)m2.x : t0 + 64;
-        for (int t = t0; t < t1; t++) {
-            if (sv >= 0 && !((m >> (t - t0)) & 1ull)) continue;
-            const float4 xj = posS[t];
-            const float r2 = dist2(xi, xj);
-            if (t == u || !(r2 <= h2)) continue;
-            sx += xj.x;
-            sy += xj.y;
-            sz += xj.z;
-            cnt++;
+    auto test = [&](int t) {
+        const float4 xj = posS[t];
+        const float r2 = dist2(xi, xj);
+        if (t == u || !(r2 <= h2)) return;
+        sx += xj.x;
+        sy += xj.y;
+        sz += xj.z;
+        cnt++;
+    };
+    const unsigned int groups = L.groups[u];
+    if (groups & VL_WINDOWS) {
+        for (unsigned int w = 0; w < groups - VL_WINDOWS; w++) {
+            const int2 se = list_window(L, n, u, (int)w);
+            for (int t = se.x; t < se.y; t++) test(t);
+        }
+    } else {
+        for (unsigned int k = 0; k < groups; k++) {
+            const int4 c = L.list[(size_t)k * n + u];
+            test(c.x);
+            test(c.y);
+            test(c.z);
+            test(c.w);
         }
     }
     bool surface = (float)cnt < countThresh;
