@@ -71,6 +71,7 @@ GridDev make_grid(const SimulationParameters& P, bool sub) {
         g.dim[a] = sub ? P.gridDimSubParticles[a] : P.gridDim[a];
     }
     g.spacing = sub ? P.gridSpacingSubParticles : P.gridSpacing;
+    g.inv = 1.0f / g.spacing;
     g.numCells = g.dim[0] * g.dim[1] * g.dim[2];
     g.cellBase = 0;
     g.rel = 0;
@@ -513,7 +514,7 @@ sph_status alloc_handle(sph_sim* s, int n, long long C) {
     SPH_CUDA(dalloc(&s->sb.sortedHash, n));
     SPH_CUDA(dalloc(&s->sb.sortedIds, n));
     SPH_CUDA(dalloc(&s->sb.workIds, n));
-    SPH_CUDA(dalloc(&s->sb.halfOffset, (size_t)C + 1));
+    SPH_CUDA(dalloc(&s->sb.halfOffset, (size_t)C + 1 + SCAN_TILE));
     SPH_CUDA(cudaMemsetAsync(s->sb.halfOffset, 0, sizeof(int) * ((size_t)C + 1), s->stream));
     // index buffers start valid (0): an entry a failed step leaves unwritten
     // still names a particle or a cell of the handle

@@ -163,6 +163,16 @@ __device__ __forceinline__ bool neighbour_r2(float r2, float h2) {
     return __float_as_uint(r2) - 1u < __float_as_uint(h2);
 }
 
+// The candidates [s, e) from cell cl of a row (its upper half on, when
+// `upperL`) to cell cr (its upper half included when `upperR`): one table
+// load an end.
+__device__ __forceinline__ void half_cells(RowTables T, int row, int cl, int cr, bool upperL, bool upperR, int& s,
+                                           int& e) {
+    s = __ldg((upperL ? T.halfOffset : T.cellOffset) + row + cl);
+    e = __ldg(upperR ? T.cellOffset + row + cr + 1 : T.halfOffset + row + cr);
+    if (e < s) e = s;
+}
+
 // Candidate range [s, e) of stencil row r (0..8: k outer, j inner).  Rows
 // outside the stencil and rows the window cut removes are empty (s == e).
 __device__ __forceinline__ void row_range(float4 xi, const Stencil& st, float h, const GridDev& g, RowTables T,
@@ -182,7 +192,7 @@ __device__ __forceinline__ void row_range(float4 xi, const Stencil& st, float h,
     const float gy = cell_gap(xi.y, y, g.origin[1], g.spacing, eps);
     const float g2 = gy * gy + gz * gz;
     if (g2 > h2) return;
-    const float inv = 1.0f / g.spacing;
+    const float inv = g.inv;
     // the reach in x: an approximate square root (relative error ~2^-22) is
     // far inside the eps margin
     float rx;
@@ -192,49 +202,30 @@ __device__ __forceinline__ void row_range(float4 xi, const Stencil& st, float h,
     const int cl = max(st.x0, (int)floorf((xl - g.origin[0]) * inv));
     const int cr = min(st.x1, (int)floorf((xr - g.origin[0]) * inv));
     if (cl > cr) return;
-    const int a0 = __ldg(T.cellOffset + row + cl), a1 = __ldg(T.cellOffset + row + cl + 1);
-    const int b0 = __ldg(T.cellOffset + row + cr), b1 = __ldg(T.cellOffset + row + cr + 1);
-    const float midL = g.origin[0] + ((float)cl + 0.5f) * g.spacing;
-    const float midR = g.origin[0] + ((float)cr + 0.5f) * g.spacing;
-    s = a0;
-    e = b1;
-    if (xl >= midL) s = min(max(__ldg(T.halfOffset + row + cl), a0), a1);
-    if (xr < midR) e = min(max(__ldg(T.halfOffset + row + cr), b0), b1);
-    if (e < s) e = s;
+    half_cells(T, row, cl, cr, xl >= g.origin[0] + ((float)cl + 0.5f) * g.spacing,
+               xr >= g.origin[0] + ((float)cr + 0.5f) * g.spacing, s, e);
 }
 
-// Candidate window [s, e) of the grid row (y, z) for a sphere of radius R
-// around xi: the row is skipped when its (y, z) cell rectangle lies farther
-// than R, and otherwise cut to the half-cells in x that the sphere reaches at
-// that gap, clamped to the grid (not to the 27-cell stencil: R may exceed a
-// cell).  The same margins as row_range, so every particle within R is a
-// candidate.  Used to build the reused neighbour lists.
-__device__ __forceinline__ bool row_window(float4 xi, int y, int z, float R, float eps, const GridDev& g,
+// Candidate window [s, e) of the grid row (y, z) at squared gap g2 from the
+// particle, for a sphere of radius R around it: cut to the half-cells in x
+// that the sphere reaches at that gap, clamped to the grid (not to the
+// 27-cell stencil: R may exceed a cell).  The same margins as row_range, so
+// every particle within R is a candidate.  Used to build the reused
+// neighbour lists.
+__device__ __forceinline__ bool row_window(float4 xi, int y, int z, float R2, float g2, float eps, const GridDev& g,
                                            RowTables T, int& s, int& e) {
     s = e = 0;
-    const float R2 = R * R;
-    const float gz = cell_gap(xi.z, z, g.origin[2], g.spacing, eps);
-    const float gy = cell_gap(xi.y, y, g.origin[1], g.spacing, eps);
-    const float g2 = gy * gy + gz * gz;
     if (g2 > R2) return false;
-    const float inv = 1.0f / g.spacing;
     float rx;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(rx) : "f"(R2 - g2));
     rx += eps;
     const float xl = xi.x - rx, xr = xi.x + rx;
-    const int cl = max(0, (int)floorf((xl - g.origin[0]) * inv));
-    const int cr = min(g.dim[0] - 1, (int)floorf((xr - g.origin[0]) * inv));
+    const int cl = max(0, (int)floorf((xl - g.origin[0]) * g.inv));
+    const int cr = min(g.dim[0] - 1, (int)floorf((xr - g.origin[0]) * g.inv));
     if (cl > cr) return false;
-    const int row = g.cellBase + g.dim[0] * (g.dim[1] * z + y);
-    const int a0 = __ldg(T.cellOffset + row + cl), a1 = __ldg(T.cellOffset + row + cl + 1);
-    const int b0 = __ldg(T.cellOffset + row + cr), b1 = __ldg(T.cellOffset + row + cr + 1);
-    const float midL = g.origin[0] + ((float)cl + 0.5f) * g.spacing;
-    const float midR = g.origin[0] + ((float)cr + 0.5f) * g.spacing;
-    s = a0;
-    e = b1;
-    if (xl >= midL) s = min(max(__ldg(T.halfOffset + row + cl), a0), a1);
-    if (xr < midR) e = min(max(__ldg(T.halfOffset + row + cr), b0), b1);
-    if (e < s) e = s;
+    half_cells(T, g.cellBase + g.dim[0] * (g.dim[1] * z + y), cl, cr,
+               xl >= g.origin[0] + ((float)cl + 0.5f) * g.spacing, xr >= g.origin[0] + ((float)cr + 0.5f) * g.spacing, s,
+               e);
     return e > s;
 }
 
@@ -246,9 +237,8 @@ __device__ __forceinline__ int2 list_window(const NeighbourLists& L, int n, int 
 
 // The cell range [lo, hi] of axis `a` that [p - r, p + r] touches, clamped to the grid.
 __device__ __forceinline__ void cell_span(float p, float r, const GridDev& g, int a, int& lo, int& hi) {
-    const float inv = 1.0f / g.spacing;
-    lo = max(0, (int)floorf((p - r - g.origin[a]) * inv));
-    hi = min(g.dim[a] - 1, (int)floorf((p + r - g.origin[a]) * inv));
+    lo = max(0, (int)floorf((p - r - g.origin[a]) * g.inv));
+    hi = min(g.dim[a] - 1, (int)floorf((p + r - g.origin[a]) * g.inv));
 }
 
 // ---------------------------------------------------------------------------
@@ -343,7 +333,7 @@ __device__ __forceinline__ void row_range_rel(float4 xi, int3 c, const Stencil& 
     const float gy = cell_gap(xi.y, 0, dyo, g.spacing, eps);
     const float g2 = gy * gy + gz * gz;
     if (g2 > h2) return;
-    const float inv = 1.0f / g.spacing;
+    const float inv = g.inv;
     // the reach in x: an approximate square root (relative error ~2^-22) is
     // far inside the eps margin
     float rx;
@@ -353,15 +343,8 @@ __device__ __forceinline__ void row_range_rel(float4 xi, int3 c, const Stencil& 
     const int cl = max(st.x0, c.x + (int)floorf(xl * inv));
     const int cr = min(st.x1, c.x + (int)floorf(xr * inv));
     if (cl > cr) return;
-    const int a0 = __ldg(T.cellOffset + row + cl), a1 = __ldg(T.cellOffset + row + cl + 1);
-    const int b0 = __ldg(T.cellOffset + row + cr), b1 = __ldg(T.cellOffset + row + cr + 1);
-    const float midL = ((float)(cl - c.x) + 0.5f) * g.spacing;
-    const float midR = ((float)(cr - c.x) + 0.5f) * g.spacing;
-    s = a0;
-    e = b1;
-    if (xl >= midL) s = min(max(__ldg(T.halfOffset + row + cl), a0), a1);
-    if (xr < midR) e = min(max(__ldg(T.halfOffset + row + cr), b0), b1);
-    if (e < s) e = s;
+    half_cells(T, row, cl, cr, xl >= ((float)(cl - c.x) + 0.5f) * g.spacing,
+               xr >= ((float)(cr - c.x) + 0.5f) * g.spacing, s, e);
 }
 
 __device__ __forceinline__ void kahan_add(float& sum, float& comp, float term) {

@@ -20,6 +20,7 @@ enum : unsigned int {
 struct GridDev {
     float origin[3];
     float spacing;
+    float inv;     // 1 / spacing
     int dim[3];
     int numCells;
     int cellBase;  // first global cell index of this grid (batched scenes; else 0)
@@ -80,7 +81,6 @@ struct SortBuffers {
     int* sortedIds;           // [n]   the reference's permutation (cell, id)
     int* workIds;             // [n]   the working order (cell, x, id) of the sorted arrays
     int* halfOffset;          // [C+1] first working index of each cell's upper x-half
-                              //       (meaningful for occupied cells only)
     unsigned long long* scanFlags;  // decoupled look-back tile states
     unsigned int* tileCounter;
     int maxTiles;
@@ -120,7 +120,7 @@ struct TwoScaleDev {
 // Per-row lookup tables of the neighbour search.
 struct RowTables {
     const int* cellOffset;  // [C+1]
-    const int* halfOffset;  // [C+1], valid for occupied cells
+    const int* halfOffset;  // [C+1]
     const SceneDev* scenes; // batched handles: per-scene grids, constants, maps (else NULL)
     const int* skip;        // as SortBuffers::skip, read by the density stage only
 };

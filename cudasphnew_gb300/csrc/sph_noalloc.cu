@@ -218,6 +218,7 @@ extern "C" sph_status sph_cell_tables_noalloc(const SimulationParameters* params
         g.dim[a] = params->gridDim[a];
     }
     g.spacing = params->gridSpacing;
+    g.inv = 1.0f / g.spacing;
     g.numCells = g.dim[0] * g.dim[1] * g.dim[2];
     g.cellBase = 0;
     const NaView v = na_view(base);

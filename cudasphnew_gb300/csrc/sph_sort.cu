@@ -239,6 +239,8 @@ constexpr unsigned long long FLAG_AGG = 1ull << 32;
 constexpr unsigned long long FLAG_INC = 2ull << 32;
 constexpr int SPIN_LIMIT = 1 << 22;
 
+// `half` gets the same offsets: an empty cell's upper half starts where the
+// cell does; the rank pass writes the occupied cells' own.
 // `waitLimit` bounds each spin (polls); a negative limit abandons every wait
 // at its first poll (a test of the give-up path: every tile then takes its
 // predecessors as zero).  A tile that gives up latches STATUS_DEVICE_WAIT and
@@ -246,7 +248,7 @@ constexpr int SPIN_LIMIT = 1 << 22;
 // offset stays within [0, n] and every index derived from the offsets stays
 // inside its buffer (the step's results are then unspecified and reported).
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, unsigned long long* flags,
+k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, int* __restrict__ half, unsigned long long* flags,
             unsigned int* tileCounter, unsigned int* status, const int* __restrict__ skip, int waitLimit,
             const unsigned int* __restrict__ sortFlag) {
     // every block alike: no tile is taken, none waited on
@@ -368,11 +370,15 @@ k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, unsigned lo
             o.w = run;
             run += v[4 * c + 3];
             *reinterpret_cast<int4*>(out + base + 4 * c) = o;
+            if (half) *reinterpret_cast<int4*>(half + base + 4 * c) = o;
         }
     } else {
 #pragma unroll
         for (int k = 0; k < SCAN_ITEMS; k++) {
-            if (base + k < total) out[base + k] = run;
+            if (base + k < total) {
+                out[base + k] = run;
+                if (half) half[base + k] = run;
+            }
             run += v[k];
         }
     }
@@ -393,7 +399,7 @@ void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaSt
     int tiles = (total + SCAN_TILE - 1) / SCAN_TILE;
     // tile counter (first 16 bytes) and the tile states that follow it
     cudaMemsetAsync(sb.tileCounter, 0, 16 + sizeof(unsigned long long) * (size_t)tiles, s);
-    k_cell_scan<<<tiles, SCAN_THREADS, 0, s>>>(total, sb.cnt, sb.cellOffset, sb.scanFlags,
+    k_cell_scan<<<tiles, SCAN_THREADS, 0, s>>>(total, sb.cnt, sb.cellOffset, sb.halfOffset, sb.scanFlags,
                                                sb.tileCounter, status, sb.skip, scan_wait_limit(), sort_flag(L));
 }
 
@@ -557,6 +563,7 @@ void launch_rebuild_tables(int n, const float4* posS, const int* workIds, const 
                            SortBuffers sb, float4* scratch, unsigned int* status, cudaStream_t s) {
     if (n <= 0) return;
     sb.skip = nullptr;
+    sb.halfOffset = nullptr;  // stays the working order's
     k_unsort_positions<<<(n + 255) / 256, 256, 0, s>>>(n, posS, workIds, slotScene, scratch);
     launch_hash_count(n, scratch, g, sb, status, s, nullptr);
     launch_cell_scan(g.numCells, sb, status, s, nullptr);

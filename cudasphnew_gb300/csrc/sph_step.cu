@@ -31,6 +31,62 @@ namespace sph {
 // Branch-free poly6 accumulation: max(h^2 - r^2, 0)^3.  Writes
 // (rho, p, p/rho^2, 1/rho) for the force stage.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ bool within_r2(float r2, float R2) {  // r2 >= 0 or NaN
+    return __float_as_uint(r2) <= __float_as_uint(R2);
+}
+
+// Up to 32 candidates of a row from slot `base`: their density terms added to
+// rs one after the other, and the bits of those within h (bit k: candidate
+// base + k), with SKIN also of those within R.  Four at a time, their loads
+// in flight together and their bits put together from constants (230 against
+// 254 us for the list build of a million particles, 21 against 27 at 16,384).
+// REL: positions are cell-relative and moved into particle i's frame.
+template <bool REL, bool SKIN>
+__device__ __forceinline__ void row_tests(const float4* __restrict__ posS, int base, int c, float4 xi, float h2,
+                                          float R2, int cx, float dyo, float dzo, float spacing, float& rs,
+                                          unsigned int& mR, unsigned int& mh) {
+    mR = mh = 0u;
+    auto at = [&](const float4* p) {
+        const float4 x = __ldg(p);
+        return REL ? rel_in_frame(x, cx, dyo, dzo, spacing) : x;
+    };
+    const float4* p = posS + base;
+    int k = 0;
+#pragma unroll 1
+    for (; k + 4 <= c; k += 4, p += 4) {
+        const float4 x0 = at(p), x1 = at(p + 1), x2 = at(p + 2), x3 = at(p + 3);
+        const float r0 = dist2(xi, x0), r1 = dist2(xi, x1), r2 = dist2(xi, x2), r3 = dist2(xi, x3);
+        const float w0 = fmaxf(h2 - r0, 0.f), w1 = fmaxf(h2 - r1, 0.f);
+        const float w2 = fmaxf(h2 - r2, 0.f), w3 = fmaxf(h2 - r3, 0.f);
+        rs = fmaf(w0 * w0, w0, rs);
+        rs = fmaf(w1 * w1, w1, rs);
+        rs = fmaf(w2 * w2, w2, rs);
+        rs = fmaf(w3 * w3, w3, rs);
+        unsigned int a = 0u, b = 0u;
+        if (SKIN) {
+            if (within_r2(r0, R2)) a = 1u;
+            if (within_r2(r1, R2)) a |= 2u;
+            if (within_r2(r2, R2)) a |= 4u;
+            if (within_r2(r3, R2)) a |= 8u;
+            mR |= a << k;
+        }
+        if (neighbour_r2(r0, h2)) b = 1u;
+        if (neighbour_r2(r1, h2)) b |= 2u;
+        if (neighbour_r2(r2, h2)) b |= 4u;
+        if (neighbour_r2(r3, h2)) b |= 8u;
+        mh |= b << k;
+    }
+#pragma unroll 1
+    for (; k < c; k++, p++) {
+        const float r2 = dist2(xi, at(p));
+        const float w = fmaxf(h2 - r2, 0.f);
+        rs = fmaf(w * w, w, rs);
+        if (SKIN) mR |= (within_r2(r2, R2) ? 1u : 0u) << k;
+        mh |= (neighbour_r2(r2, h2) ? 1u : 0u) << k;
+    }
+}
+
+
 // With REL the positions are cell-relative: every neighbour is moved into
 // particle i's cell frame before its distance is taken.
 // Occupancy: 40 registers (six 256-thread blocks per SM) cost no spills
@@ -52,38 +108,25 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
     const Stencil st = REL ? stencil_rel(xi, ci, ph.h, g) : stencil(xi, ph.h, g);
     const float h2 = ph.h2;
     float sum = 0.f, comp = 0.f;
-#pragma unroll
+#pragma unroll 1
     for (int r = 0; r < 9; r++) {
         int s, e;
         float dyo = 0.f, dzo = 0.f;
         if (REL) row_range_rel(xi, ci, st, ph.h, g, T, window != 0, r, s, e, dyo, dzo);
         else row_range(xi, st, ph.h, g, T, window != 0, r, s, e);
         float rs = 0.f;
-        // neighbour bits, first candidate in the highest bit used (one
-        // multiply-add per candidate), turned around after the row; two
-        // candidates per loop turn (176 -> 172 us per million particles;
-        // four gain nothing more)
-        unsigned int m = 0u;
-#pragma unroll 2
-        for (int t = s; t < e; t++) {
-            float4 xj = __ldg(posS + t);
-            if (REL) xj = rel_in_frame(xj, ci.x, dyo, dzo, g.spacing);
-            const float r2 = dist2(xi, xj);
-            const float w = fmaxf(h2 - r2, 0.f);
-            rs = fmaf(w * w, w, rs);
-            if (EMIT) m = m * 2u + (neighbour_r2(r2, h2) ? 1u : 0u);
-        }
+        unsigned int m = 0u, mR;
+        for (int base = s; base < e; base += 32)
+            row_tests<REL, false>(posS, base, min(32, e - base), xi, h2, 0.f, ci.x, dyo, dzo, g.spacing, rs, mR, m);
         if (KAHAN) {
             if (rs > 0.f) kahan_add(sum, comp, rs);
         } else {
             sum += rs;
         }
         if (EMIT) {
-            const int c = e - s;
-            const bool fits = c <= 32;
-            const unsigned int bits = (fits && c > 0) ? __brev(m) >> (32 - c) : 0u;  // bit k: candidate s + k
+            const bool fits = e - s <= 32;  // bit k: candidate s + k
             M.start[(size_t)r * n + i] = fits ? s : (s | (int)0x80000000);
-            M.mask[(size_t)r * n + i] = fits ? bits : (unsigned int)e;
+            M.mask[(size_t)r * n + i] = fits ? m : (unsigned int)e;
         }
     }
     float rho = (KAHAN ? __fsub_rn(sum, comp) : sum) * ph.poly6m;
@@ -100,23 +143,18 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
 // ---------------------------------------------------------------------------
 // Density over reused neighbour lists (sph_options.neighbourSkin).
 //
-// Build form (steps that build the lists): the reference's 3 x 3 stencil
-// rows first, in its order, then the further rows the skin sphere of radius R
-// reaches; each row's window at R is walked in the working order.  The
-// reference's rows give the density terms, summed as in k_density (candidates
+// Build form (steps that build the lists): every row that the skin sphere of
+// radius R reaches, in the reference's order, its window at R walked in the
+// working order.  The reference's own 3 x 3 rows give the density terms, summed as in k_density (candidates
 // beyond h add exactly nothing, so the row sums are the same), and this
 // step's neighbours by row for the force stage; every row gives its
 // candidates within R to the particle's list.  A step that searches without
 // building (VL_SEARCHES) takes windows at h and records those.
 //
 // A row is tested 32 candidates at a time into two bit masks (within R,
-// within h; one multiply-add each), and only the set bits are appended: the
-// append costs ten times the test and a third of the candidates pass.
+// within h), and only the set bits are appended: an append costs as much as a
+// test and a quarter of the candidates pass.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool within_r2(float r2, float R2) {  // r2 >= 0 or NaN
-    return __float_as_uint(r2) <= __float_as_uint(R2);
-}
-
 // BATCH: the slot's scene supplies grid, constants, maps, R and the scene's
 // own decision.
 template <bool KAHAN, bool BATCH>
@@ -144,26 +182,33 @@ __device__ __forceinline__ void density_build_one(int i, int n, float4* posS, fl
         count++;
         if ((count & 3) == 0 && count <= VL_CAP) L.list[(size_t)((count >> 2) - 1) * n + i] = group;
     };
-    // row (y, z); slot >= 0: one of the reference's rows, recorded even when empty
-    auto visit = [&](int y, int z, int slot) {
-        int s0 = 0, e0 = 0;
-        if (y >= 0) row_window(xi, y, z, R, eps, g, T, s0, e0);
+    // every row the sphere reaches, in the reference's order (k outer, j inner)
+    const int y1 = min(st.y1, st.y0 + 2), z1 = min(st.z1, st.z0 + 2);
+    int ya, yb, za, zb;
+    cell_span(xi.y, R + eps, g, 1, ya, yb);
+    cell_span(xi.z, R + eps, g, 2, za, zb);
+    const float reach2 = R * R;
+    auto rows = [&](auto&& row) {
+#pragma unroll 1
+        for (int z = za; z <= zb; z++) {
+            const float gz = cell_gap(xi.z, z, g.origin[2], g.spacing, eps);
+#pragma unroll 1
+            for (int y = ya; y <= yb; y++) {
+                const float gy = cell_gap(xi.y, y, g.origin[1], g.spacing, eps);
+                int s, e;
+                if (row_window(xi, y, z, reach2, gy * gy + gz * gz, eps, g, T, s, e)) row(y, z, s, e);
+            }
+        }
+    };
+    unsigned int seen = 0u;  // the reference's rows that were walked
+    rows([&](int y, int z, int s0, int e0) {
+        const bool inner = z >= st.z0 && z <= z1 && y >= st.y0 && y <= y1;
         float rs = 0.f;
         int first = -1, last = -1;
         unsigned int m = 0u;  // neighbours within h, bit t - first
         for (int base = s0; base < e0; base += 32) {
-            const int c = min(32, e0 - base);
-            unsigned int mR = 0u, mh = 0u;  // first candidate in the highest bit used, turned around below
-#pragma unroll 2
-            for (int t = base; t < base + c; t++) {
-                const float r2 = dist2(xi, __ldg(posS + t));
-                const float w = fmaxf(h2 - r2, 0.f);
-                rs = fmaf(w * w, w, rs);
-                mR = mR * 2u + (within_r2(r2, R2) ? 1u : 0u);
-                mh = mh * 2u + (neighbour_r2(r2, h2) ? 1u : 0u);
-            }
-            mR = lists ? __brev(mR) >> (32 - c) : 0u;
-            mh = __brev(mh) >> (32 - c);
+            unsigned int mR, mh;
+            row_tests<false, true>(posS, base, min(32, e0 - base), xi, h2, R2, 0, 0.f, 0.f, 0.f, rs, mR, mh);
             if (mh) {
                 if (first < 0) {
                     const int k = __ffs(mh) - 1;
@@ -174,53 +219,41 @@ __device__ __forceinline__ void density_build_one(int i, int n, float4* posS, fl
                 }
                 last = base + 31 - __clz(mh);
             }
+            if (!lists) mR = 0u;
             while (mR) {
                 const int k = __ffs(mR) - 1;
                 mR &= mR - 1u;
                 append(base + k);
             }
         }
-        if (slot < 0) return;
+        if (!inner) return;
         if (KAHAN) {
             if (rs > 0.f) kahan_add(sum, comp, rs);
         } else {
             sum += rs;
         }
         const bool fits = last - first < 32;
-        const size_t at = (size_t)slot * n + i;
-        M.start[at] = first < 0 ? 0 : fits ? first : (first | (int)0x80000000);
-        M.mask[at] = fits ? m : (unsigned int)(last + 1);
-    };
-    // the reference's rows (k_density's order), then the rest within R
-    const int y1 = min(st.y1, st.y0 + 2), z1 = min(st.z1, st.z0 + 2);
-    int ya, yb, za, zb;
-    cell_span(xi.y, R + eps, g, 1, ya, yb);
-    cell_span(xi.z, R + eps, g, 2, za, zb);
-    auto rows = [&](auto&& row) {
-#pragma unroll 1
-        for (int r = 0; r < 9; r++) {
-            const int z = st.z0 + r / 3, y = st.y0 + r % 3;
-            row(z <= z1 && y <= y1 ? y : -1, z, r);
-        }
-        if (!lists) return;
-#pragma unroll 1
-        for (int z = za; z <= zb; z++)
-#pragma unroll 1
-            for (int y = ya; y <= yb; y++)
-                if (z < st.z0 || z > z1 || y < st.y0 || y > y1) row(y, z, -1);
-    };
-    rows(visit);
+        const int slot = 3 * (z - st.z0) + y - st.y0;
+        seen |= 1u << slot;
+        M.start[(size_t)slot * n + i] = first < 0 ? 0 : fits ? first : (first | (int)0x80000000);
+        M.mask[(size_t)slot * n + i] = fits ? m : (unsigned int)(last + 1);
+    });
+    for (unsigned int none = ~seen & 0x1ffu; none; none &= none - 1u) {
+        const size_t at = (size_t)(__ffs(none) - 1) * n + i;
+        M.start[at] = 0;
+        M.mask[at] = 0u;
+    }
     if (lists && count <= VL_CAP) {
         L.groups[i] = (unsigned char)((count + 3) >> 2);
         while (count & 3) append(n);
     } else {
         // too many for the list, or no list to build: the rows' windows
         int w = 0;
-        rows([&](int y, int z, int) {
-            int s0 = 0, e0 = 0;
-            if (y < 0 || w >= VL_ROWS || !row_window(xi, y, z, R, eps, g, T, s0, e0)) return;
-            reinterpret_cast<int2*>(L.list + (size_t)(w >> 1) * n + i)[w & 1] = make_int2(s0, e0);
-            w++;
+        rows([&](int, int, int s0, int e0) {
+            if (w < VL_ROWS) {
+                reinterpret_cast<int2*>(L.list + (size_t)(w >> 1) * n + i)[w & 1] = make_int2(s0, e0);
+                w++;
+            }
         });
         L.groups[i] = (unsigned char)(VL_WINDOWS + w);
     }
