@@ -172,7 +172,7 @@ void free_all(sph_sim* s) {
     for (cudaEvent_t e : s->events) cudaEventDestroy(e);
     void* ptrs[] = {s->pos, s->vel, s->posS, s->velS, s->rho4S, s->accS, s->sb.cnt, s->sb.cellOffset,
                     s->sb.keySlot, s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds,
-                    s->sb.halfOffset, s->scanBlock,
+                    s->sb.halfOffset, s->sb.front, s->scanBlock,
                     s->status, s->staging, s->map4, s->mapDist, s->rowStart, s->rowMask, s->diagBuf,
                     s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.posB,
                     s->vl.flags, s->vl.slotScene};
@@ -326,6 +326,22 @@ sph_status alloc_lists(sph_sim* s) {
     return SPH_OK;
 }
 
+// The front of a step; with stage events its phases as launches of their own,
+// so that each can be timed.
+static void enqueue_front(sph_sim* s, const float4* pos, const float4* vel, const GridDev& g, const NeighbourLists* L,
+                          cudaEvent_t* ev) {
+    cudaStream_t st = s->stream;
+    if (!ev) {
+        launch_front(s->n, pos, vel, g, s->sb, s->posS, s->velS, s->status, st, L);
+        return;
+    }
+    const int phases[4] = {FRONT_HASH, FRONT_SUM | FRONT_SCAN, FRONT_SCATTER, FRONT_RANK};
+    for (int k = 0; k < 4; k++) {
+        cudaEventRecord(ev[ST_HASH + k], st);
+        launch_front(s->n, pos, vel, g, s->sb, s->posS, s->velS, s->status, st, L, phases[k]);
+    }
+}
+
 // A plain step over the reused neighbour lists: the decision, the
 // reference's hash, sort and cell tables when some scene builds (a step that
 // builds nothing skips them; sph_read_cells builds its tables on demand),
@@ -337,19 +353,9 @@ static void enqueue_lists(sph_sim* s, const GridDev& g, const PhysDev& ph, int c
     auto mark = [&](int k) {
         if (ev) cudaEventRecord(ev[k], st);
     };
-    mark(ST_HASH);
-    launch_hash_count(n, s->pos, g, s->sb, s->status, st, &s->vl);
-    mark(ST_SCAN);
-    launch_cell_scan(g.numCells, s->sb, s->status, st, &s->vl);
-    mark(ST_SCATTER);
-    launch_scatter(n, s->sb, st, s->status, &s->vl);
-    mark(ST_RANK);
-    launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, &s->vl, s->status);
+    enqueue_front(s, s->pos, s->vel, g, &s->vl, ev);
     mark(ST_DENSITY);
-    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, true,
-                         true, st);
-    // the sorted copies are now this step's own: a reuse the audit granted is used up
-    cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
+    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, st);
     mark(ST_FORCE);
     launch_force_lists(n, s->posS, s->velS, s->rho4S, s->sb.workIds, ph, s->map, collide, s->vl, masks_of(s), s->pos,
                        s->vel, s->accS, s->cfg, st, s->sb.scenes);
@@ -370,19 +376,13 @@ void enqueue_coarse(sph_sim* s, const GridDev& g, const PhysDev& ph, int collide
     auto mark = [&](int k) {
         if (ev) cudaEventRecord(ev[k], st);
     };
-    mark(ST_HASH);
-    launch_hash_count(n, s->pos, g, s->sb, s->status, st);
-    mark(ST_SCAN);
-    launch_cell_scan(g.numCells, s->sb, s->status, st);
-    mark(ST_SCATTER);
-    launch_scatter(n, s->sb, st, s->status);
-    mark(ST_RANK);
-    launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, nullptr, s->status);
+    enqueue_front(s, s->pos, s->vel, g, nullptr, ev);
     mark(ST_DENSITY);
     // density and forces read the sorted copies only
     launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, cfg, st);
-    // the sorted copies are now this step's own: a reuse the audit granted is used up
-    cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
+    // the sorted copies are now this step's own: a reuse the audit granted is
+    // used up (without a corrector there is no audit)
+    if (s->corr) cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
     mark(ST_FORCE);
     if (!force) return;
     launch_force(n, s->posS, s->velS, s->rho4S, s->sb.workIds, rows_of(s), g, ph, s->map, collide, s->rowStart,
@@ -397,10 +397,7 @@ void enqueue_density_only(sph_sim* s, const float4* pos, const float4* vel, bool
     GridDev g = grid_of(s);
     PhysDev ph = make_phys(s->P, s->O);
     mark_tables_current(s);
-    launch_hash_count(n, pos, g, s->sb, s->status, st);
-    launch_cell_scan(g.numCells, s->sb, s->status, st);
-    launch_scatter(n, s->sb, st, s->status);
-    launch_rank_gather(n, s->sb, pos, vel, g, s->posS, s->velS, st, nullptr, s->status);
+    launch_front(n, pos, vel, g, s->sb, s->posS, s->velS, s->status, st);
     StepConfig cfg = s->cfg;
     cfg.forceVariant = masks ? FORCE_PRETESTED : FORCE_MASK;  // whether to record the neighbour masks
     launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, cfg, st);
@@ -411,12 +408,8 @@ void enqueue_list_density(sph_sim* s, const float4* pos, const float4* vel) {
     const int n = s->n;
     GridDev g = grid_of(s);
     PhysDev ph = make_phys(s->P, s->O);
-    launch_hash_count(n, pos, g, s->sb, s->status, st, &s->vl);
-    launch_cell_scan(g.numCells, s->sb, s->status, st, &s->vl);
-    launch_scatter(n, s->sb, st, s->status, &s->vl);
-    launch_rank_gather(n, s->sb, pos, vel, g, s->posS, s->velS, st, &s->vl, s->status);
-    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, true,
-                         true, st);
+    launch_front(n, pos, vel, g, s->sb, s->posS, s->velS, s->status, st, &s->vl);
+    launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, st);
 }
 
 void invalidate_graphs(sph_sim* s) {
@@ -524,6 +517,8 @@ sph_status alloc_handle(sph_sim* s, int n, long long C) {
     s->sb.tileCounter = reinterpret_cast<unsigned int*>(s->scanBlock);
     s->sb.scanFlags = s->scanBlock + 2;
     s->sb.maxTiles = (int)tiles;
+    SPH_CUDA(dalloc(&s->sb.front, FRONT_WORDS));
+    SPH_CUDA(cudaMemsetAsync(s->sb.front, 0, sizeof(unsigned int) * FRONT_WORDS, s->stream));
     SPH_CUDA(dalloc(&s->status, 1));
     SPH_CUDA(dalloc(&s->reuse, 1));
     s->sb.skip = s->reuse;
@@ -1451,10 +1446,7 @@ sph_status sph_autotune(sph_handle s, int reps, sph_tuning* chosen) {
     GridDev g = grid_of(s);
     PhysDev ph = make_phys(s->P, s->O);
     auto sortStages = [&]() {
-        launch_hash_count(n, s->pos, g, s->sb, s->status, st);
-        launch_cell_scan(g.numCells, s->sb, s->status, st);
-        launch_scatter(n, s->sb, st, s->status);
-        launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, nullptr, s->status);
+        launch_front(n, s->pos, s->vel, g, s->sb, s->posS, s->velS, s->status, st);
     };
     // each candidate is timed in step context: the sort stages run before
     // every timed launch, so caches hold what they hold in a real step; the
@@ -1650,7 +1642,7 @@ sph_status sph_time_kernel(sph_handle s, int stage, int reps, float* microsecond
         if (lists) {
             if (stage == ST_DENSITY)
                 launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg,
-                                     false, true, st);
+                                     st);
             else
                 launch_force_lists(n, s->posS, s->velS, s->rho4S, s->sb.workIds, ph, s->map, s->O.boxCollision,
                                    s->vl, masks_of(s), s->pos, s->vel, s->accS, s->cfg, st, s->sb.scenes);

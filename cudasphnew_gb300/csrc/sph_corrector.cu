@@ -111,6 +111,7 @@ sph_status ensure_corrector(sph_sim* s) {
     if (s->corr) return SPH_OK;
     Corrector* C = new Corrector();
     s->corr = C;
+    invalidate_graphs(s);  // steps use up a reuse an audit grants from here on
     const size_t n = (size_t)s->n;
     SPH_CUDA(dalloc(&C->master, NPARAM));
     SPH_CUDA(dalloc(&C->m1, NPARAM));
@@ -172,14 +173,8 @@ void enqueue_learned(sph_sim* s, Corrector* C) {
     StepConfig cfg = s->cfg;
     const FeatureOut fo{C->record ? C->feat : nullptr, 1, s->O.boxCollision, ph.dt};
     if (s->vlOn) {
-        launch_hash_count(n, s->pos, g, s->sb, s->status, st, &s->vl);
-        launch_cell_scan(g.numCells, s->sb, s->status, st, &s->vl);
-        launch_scatter(n, s->sb, st, s->status, &s->vl);
-        launch_rank_gather(n, s->sb, s->pos, s->vel, g, s->posS, s->velS, st, &s->vl, s->status);
-        launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), cfg, true,
-                             true, st);
-        // the sorted copies are now this step's own: a reuse the audit granted is used up
-        cudaMemsetAsync(s->reuse, 0, sizeof(int), st);
+        launch_front(n, s->pos, s->vel, g, s->sb, s->posS, s->velS, s->status, st, &s->vl);
+        launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), cfg, st);
         launch_force_learned(n, s->posS, s->velS, s->rho4S, s->sb.workIds, rows_of(s), g, ph, s->map,
                              s->O.boxCollision, s->rowStart, s->rowMask, s->pos, s->vel, s->accS, cfg, fo, mdev(C),
                              s->status, st, &s->vl);

@@ -84,6 +84,7 @@ struct SortBuffers {
     unsigned long long* scanFlags;  // decoupled look-back tile states
     unsigned int* tileCounter;
     int maxTiles;
+    unsigned int* front;      // [FRONT_WORDS] k_front's barrier and block sums, zero between launches
     const SceneDev* scenes;   // batched handles: per-scene grids (else NULL)
     const int* skip;          // when non-NULL and set on the device, the sorted copies and
                               // tables already hold the current state: the sort stages return
@@ -157,7 +158,8 @@ enum : int {
     VL_BUILD_NOW = 1,  // this step's kind, a VL_REUSES ... (decided at the start of the step)
     VL_DISP = 2,       // largest squared displacement since the build (float bits)
     VL_COUNT = 3,      // builds so far
-    VL_FLAGS = 4,
+    VL_LAST = 4,       // the kind of the step before, until this step's front is done
+    VL_FLAGS = 5,
 };
 // A step reuses the lists, builds them, or searches without building: when a
 // step has moved some particle past the rebuild distance by itself, lists
@@ -238,44 +240,30 @@ void launch_pack_aos(const float4* in, int n, float* aos, int stride, int offset
 // back to absolute (AoS with `stride` floats per particle and/or float4s).
 void launch_abs_to_rel(int n, float4* pos, GridDev g, cudaStream_t s);
 void launch_rel_to_abs(int n, const float4* pos, GridDev g, float* aos, int stride, float4* out4, cudaStream_t s);
-// With `lists`, a one-block kernel first decides whether each scene builds
-// the neighbour lists in this step (VL_BUILD_NOW) and whether the step sorts
-// (VL_SORT); the hash pass returns at once when it does not.
-void launch_hash_count(int n, const float4* pos, GridDev g, SortBuffers sb, unsigned int* status,
-                       cudaStream_t s, const NeighbourLists* lists = nullptr);
-// With `lists`, the scan and the scatter return at once in a step that
-// builds no lists (VL_SORT clear), and so does the hash pass (whose checks of
-// the state the rank pass then makes).
-void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s,
-                      const NeighbourLists* lists = nullptr);
-// With `status`, the scatter leaves its outputs as they were once a scan
-// wait has given up (STATUS_DEVICE_WAIT).
-void launch_scatter(int n, SortBuffers sb, cudaStream_t s, const unsigned int* status = nullptr,
-                    const NeighbourLists* lists = nullptr);
+// The front of a step (k_front): hash, scan, scatter, rank and gather of the
+// state (pos, vel) into the sorted copies, the permutations and the cell
+// tables.  With `lists` the kind of step is decided first, and one that sorts
+// nothing only gathers.  Parts of it: `phases`, in this order.
+enum : int { FRONT_HASH = 1, FRONT_SUM = 2, FRONT_SCAN = 4, FRONT_SCATTER = 8, FRONT_RANK = 16, FRONT_ALL = 31 };
+constexpr int FRONT_MAX_BLOCKS = 4088;
+constexpr int FRONT_WORDS = FRONT_MAX_BLOCKS + 8;
+void launch_front(int n, const float4* pos, const float4* vel, GridDev g, SortBuffers sb, float4* posS, float4* velS,
+                  unsigned int* status, cudaStream_t s, const NeighbourLists* lists = nullptr, int phases = FRONT_ALL);
+// The fine level's cell offsets (two-scale pass).
+void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s);
 // The cell tables of the sorted copies' positions (sortedHash, sortedIds,
 // cellOffset) after a step that skipped them; the working order, the sorted
 // copies and the lists stay as they are.  `scratch`: n float4.
 void launch_rebuild_tables(int n, const float4* posS, const int* workIds, const int* slotScene, GridDev g,
                            SortBuffers sb, float4* scratch, unsigned int* status, cudaStream_t s);
-// With `lists` and no build in this step, only the reference permutation is
-// ranked and the state is gathered into the kept working order (workIds).
-// With `status`, the pass leaves its outputs as they were once a scan wait
-// has given up (STATUS_DEVICE_WAIT).
-// In a step that sorts nothing (lists, VL_SORT clear) the pass only gathers
-// the state into the kept order and makes the hash pass's checks (non-finite
-// positions, positions outside the grid), latching them in `status`.
-void launch_rank_gather(int n, SortBuffers sb, const float4* pos, const float4* vel, GridDev g,
-                        float4* posS, float4* velS, cudaStream_t s, const NeighbourLists* lists = nullptr,
-                        unsigned int* status = nullptr);
 // Density stage over reused neighbour lists: the build form (the reference's
 // rows and the skin rows, recording the lists, and in M this step's
-// neighbours by row) and the list form; each returns at once unless the step
-// is of its kind.
+// neighbours by row) or the list form, as each scene's kind of step asks.
 // Besides rho4S, each particle's p/rho^2 and 1/rho go to the fourth lanes of
 // its sorted position and velocity, where the list force stage reads them.
 void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg, bool build,
-                          bool reuse, cudaStream_t s);
+                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg,
+                          cudaStream_t s);
 // After a write of the positions: the largest distance from the build
 // positions, measured afresh (the lists stay if it is within the limit).
 // (Batched handles: each particle's scene from the .w lane of its position.)

@@ -9,13 +9,13 @@
 //   accS               float4[n]  acceleration in sorted order
 //   cnt, cellOffset    int[C+1]   per-cell counts / their exclusive scan
 // The sort is a counting sort: every particle takes an arrival slot in its
-// cell with one atomic, a single-pass decoupled look-back scan turns counts
-// into cell offsets, and a rank pass orders each cell's members by particle
-// id.  The result is the permutation of a stable sort by hash -- the order
+// cell with one atomic, a scan turns counts into cell offsets, and a rank pass
+// orders each cell's members by particle id.  The result is the permutation of a stable sort by hash -- the order
 // thrust::sort_by_key produces in the reference (particle_simulation.cu:2340).
 #include <cuda/atomic>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "sph_device.cuh"
@@ -125,112 +125,8 @@ void launch_pack_aos(const float4* in, int n, float* aos, int stride, int offset
 }
 
 // ---------------------------------------------------------------------------
-// Stage 1: hash + per-cell arrival slot
-// ---------------------------------------------------------------------------
-// With BATCH the particle's scene (pos.w) supplies its grid, whose cells
-// start at that scene's cellBase in the concatenated cell space.
-// With REL the position is cell-relative and the hash comes from its packed
-// cell coordinates.
-// With reused neighbour lists the pass returns at once in a step that builds
-// none (k_list_decide has decided; the rank pass checks the state instead).
-template <bool BATCH, bool REL>
-__global__ void k_hash_count(int n, const float4* __restrict__ pos, GridDev g_, const SceneDev* __restrict__ scenes,
-                             int* __restrict__ cnt, int2* __restrict__ keySlot, unsigned int* status,
-                             const int* __restrict__ skip, const unsigned int* __restrict__ sortFlag) {
-    if ((sortFlag && !*sortFlag) || (skip && *skip)) return;
-    // one wave of blocks striding over the particles (a step that returns
-    // at once then costs one wave; the arrival order in a cell is ranked
-    // away later, so the grid shape changes no result)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 p = pos[i];
-        const GridDev& g = BATCH ? scenes[__float_as_int(p.w)].g : g_;
-        bool outside = false;
-        const bool finite = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
-        if (!finite) {
-            atomicOr(status, STATUS_NON_FINITE);
-            p = make_float4(g.origin[0], g.origin[1], g.origin[2], 0.f);
-        }
-        int h;
-        if (REL) {
-            const int3 c = finite ? rel_cell(p) : make_int3(0, 0, 0);
-            h = g.cellBase + g.dim[0] * (g.dim[1] * c.z + c.y) + c.x;
-        } else {
-            h = particle_hash(p, g, &outside);
-        }
-        if (outside) atomicOr(status, STATUS_OUT_OF_DOMAIN);
-        int slot = atomicAdd(cnt + h, 1);
-        keySlot[i] = make_int2(h, slot);
-    }
-}
-
-// Blocks of 256 threads for the striding sort passes: one full wave.
-static int stride_blocks(int n) {
-    const int want = (n + 255) / 256;
-    return std::max(1, std::min(want, device_sms() * (2048 / 256)));
-}
-
-// Reused neighbour lists: whether each scene builds them in this step (on
-// request, or when one of its particles has moved farther than the skin
-// allows since the last build, or the displacement is not finite; thread k
-// decides scene k; VL_SEARCHES in place of a build that the last step's own
-// displacement would have outrun), whether the step sorts (some scene builds) and whether
-// it leaves the cell tables stale (it does not sort).  One block.
-__global__ void k_list_decide(NeighbourLists L, const SceneDev* __restrict__ scenes) {
-    __shared__ int anyBuild;
-    if (threadIdx.x == 0) anyBuild = 0;
-    __syncthreads();
-    const int S = L.numScenes;
-    unsigned int* f = L.flags;
-    for (int k = threadIdx.x; k < S; k += blockDim.x) {
-        float lim2 = L.dispLimit2;
-        if (scenes) {
-            const float lim = 0.45f * L.skinFrac * scenes[k].ph.h;
-            lim2 = lim * lim;
-        }
-        const float d2 = __uint_as_float(f[VL_DISP * S + k]);
-        const bool asked = f[VL_BUILD * S + k] != 0u, past = !(d2 <= lim2);
-        const unsigned int last = f[VL_BUILD_NOW * S + k];
-        const unsigned int kind = asked                ? VL_BUILDS
-                                  : past               ? (last == VL_REUSES ? VL_BUILDS : VL_SEARCHES)
-                                  : last == VL_SEARCHES ? VL_BUILDS
-                                                        : VL_REUSES;
-        f[VL_BUILD_NOW * S + k] = kind;
-        f[VL_BUILD * S + k] = 0u;
-        if (kind != VL_REUSES) {
-            f[VL_DISP * S + k] = 0u;
-            if (kind == VL_BUILDS) f[VL_COUNT * S + k] += 1u;
-            anyBuild = 1;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        f[VL_FLAGS * S + VL_SORT] = anyBuild ? 1u : 0u;
-        f[VL_FLAGS * S + VL_STALE] = anyBuild ? 0u : 1u;
-    }
-}
-
-static const unsigned int* sort_flag(const NeighbourLists* L) {
-    return L ? L->flags + VL_FLAGS * L->numScenes + VL_SORT : nullptr;
-}
-
-void launch_hash_count(int n, const float4* pos, GridDev g, SortBuffers sb, unsigned int* status,
-                       cudaStream_t s, const NeighbourLists* L) {
-    if (n <= 0) return;
-    if (L) k_list_decide<<<1, 256, 0, s>>>(*L, sb.scenes);
-    const unsigned int* sf = sort_flag(L);
-    const int grid = stride_blocks(n);
-    if (sb.scenes)
-        k_hash_count<true, false><<<grid, 256, 0, s>>>(n, pos, g, sb.scenes, sb.cnt, sb.keySlot, status, sb.skip, sf);
-    else if (g.rel)
-        k_hash_count<false, true><<<grid, 256, 0, s>>>(n, pos, g, nullptr, sb.cnt, sb.keySlot, status, sb.skip,
-                                                       nullptr);
-    else
-        k_hash_count<false, false><<<grid, 256, 0, s>>>(n, pos, g, nullptr, sb.cnt, sb.keySlot, status, sb.skip, sf);
-}
-
-// ---------------------------------------------------------------------------
-// Stage 2: exclusive scan of the C+1 cell counts into cell offsets, one pass
-// with decoupled look-back (Merrill & Garland).  Counts are cleared as they
+// The fine level's scan (two-scale pass): exclusive scan of the C+1 cell
+// counts into cell offsets, one pass with decoupled look-back (Merrill & Garland).  Counts are cleared as they
 // are read, ready for the next step.  Tiles take their index from an atomic
 // counter, so every tile a block waits on has already started; each wait is
 // bounded and latches STATUS_DEVICE_WAIT if it ever gives up.
@@ -239,8 +135,6 @@ constexpr unsigned long long FLAG_AGG = 1ull << 32;
 constexpr unsigned long long FLAG_INC = 2ull << 32;
 constexpr int SPIN_LIMIT = 1 << 22;
 
-// `half` gets the same offsets: an empty cell's upper half starts where the
-// cell does; the rank pass writes the occupied cells' own.
 // `waitLimit` bounds each spin (polls); a negative limit abandons every wait
 // at its first poll (a test of the give-up path: every tile then takes its
 // predecessors as zero).  A tile that gives up latches STATUS_DEVICE_WAIT and
@@ -248,11 +142,8 @@ constexpr int SPIN_LIMIT = 1 << 22;
 // offset stays within [0, n] and every index derived from the offsets stays
 // inside its buffer (the step's results are then unspecified and reported).
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, int* __restrict__ half, unsigned long long* flags,
-            unsigned int* tileCounter, unsigned int* status, const int* __restrict__ skip, int waitLimit,
-            const unsigned int* __restrict__ sortFlag) {
-    // every block alike: no tile is taken, none waited on
-    if ((skip && *skip) || (sortFlag && !*sortFlag)) return;
+k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, unsigned long long* flags,
+            unsigned int* tileCounter, unsigned int* status, int waitLimit) {
     __shared__ int s_tile;
     __shared__ int s_warp[SCAN_THREADS / 32];
     __shared__ int s_prefix;
@@ -370,21 +261,17 @@ k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, int* __rest
             o.w = run;
             run += v[4 * c + 3];
             *reinterpret_cast<int4*>(out + base + 4 * c) = o;
-            if (half) *reinterpret_cast<int4*>(half + base + 4 * c) = o;
         }
     } else {
 #pragma unroll
         for (int k = 0; k < SCAN_ITEMS; k++) {
-            if (base + k < total) {
-                out[base + k] = run;
-                if (half) half[base + k] = run;
-            }
+            if (base + k < total) out[base + k] = run;
             run += v[k];
         }
     }
 }
 
-// The look-back's poll limit: SPIN_LIMIT, or the integer in the environment
+// The poll limit of a wait: SPIN_LIMIT, or the integer in the environment
 // variable SPH_SCAN_WAIT_LIMIT (read at each launch; a captured step graph
 // keeps the value it was captured with).  Tests set it to exercise the
 // give-up path; -1 abandons every wait at once.
@@ -394,142 +281,396 @@ static int scan_wait_limit() {
     return (int)strtol(e, nullptr, 10);
 }
 
-void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s, const NeighbourLists* L) {
+void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s) {
     int total = numCells + 1;
     int tiles = (total + SCAN_TILE - 1) / SCAN_TILE;
     // tile counter (first 16 bytes) and the tile states that follow it
     cudaMemsetAsync(sb.tileCounter, 0, 16 + sizeof(unsigned long long) * (size_t)tiles, s);
-    k_cell_scan<<<tiles, SCAN_THREADS, 0, s>>>(total, sb.cnt, sb.cellOffset, sb.halfOffset, sb.scanFlags,
-                                               sb.tileCounter, status, sb.skip, scan_wait_limit(), sort_flag(L));
+    k_cell_scan<<<tiles, SCAN_THREADS, 0, s>>>(total, sb.cnt, sb.cellOffset, sb.scanFlags, sb.tileCounter, status,
+                                               scan_wait_limit());
 }
 
 // ---------------------------------------------------------------------------
-// Stage 3: scatter ids into their cell segments (arrival order)
+// The front of a step: hash, cell offsets, scatter, rank and gather, in one
+// cooperative launch whose phases are set apart by grid barriers.  As separate
+// kernels (six, with a memset and those that returned at once) a step spent
+// more on their launches than on their work: a searching step of 131,071
+// particles 77 -> 64 us, one of 16,384 that reuses its lists 29 -> 19 us.
+//
+//   hash     every particle takes an arrival slot in its cell with one atomic;
+//   scan     the C+1 counts into cell offsets: every block sums its stretch of
+//            cells, then adds the sums of the stretches before it and scans
+//            its own; the counts are cleared as they are read;
+//   scatter  ids to their cell's segment, in arrival order;
+//   rank     orders each cell's members and gathers the state.  Two orders
+//            come out of one pass over the cell segment:
+//              by particle id -> sortedIds, the reference's permutation
+//                 (stable sort by hash, particle_simulation.cu:2340), for the API;
+//              by (x, id)     -> workIds, the order the neighbour kernels use:
+//                 a cell's members sorted by x, so the lower and upper x-halves
+//                 of a cell are two contiguous ranges (halfOffset: the first
+//                 index with x >= the cell's mid-plane; an empty cell's is
+//                 where the cell starts).
+//            Ranks count the smaller keys in the segment; x is compared
+//            through its order-preserving integer image so the order is total
+//            (NaN included).
+//
+// The grid is small on purpose: a cooperative grid waits until all of it fits
+// on the GPU, which the kernels of other handles (streams) then leave idle.
+// One block an SM, two above FRONT_WIDE particles.  Three handles stepped in
+// turn, us a step with 1 / 2 / 3 blocks an SM / five ordinary launches, and in
+// brackets one handle alone: 262,144 particles searching 75 / 82 / 96 / 83
+// [119 / 116 / 117 / 120]; reusing lists 56 / 59 / 67 / 64 [74 / 73 / 74 / 86];
+// 1,048,576 reusing lists 198 / 201 / 208 / 210 [248 / 238 / 236 / 249].
+//
+// With reused neighbour lists each scene's kind of step (VL_REUSES ...) is
+// decided first, by every block from the same flags.  Where no scene sorts
+// there is nothing but a gather of the state into the kept order (workIds),
+// with the hash's checks of each position; in a step that sorts, a scene that
+// reuses its lists has its ids ranked and its state gathered into its kept order.
+//
+// Every wait is bounded.  A block whose wait gives up latches
+// STATUS_DEVICE_WAIT and leaves; the rest follow, and the last to leave clears
+// the counts and asks for new lists: every offset and id left behind is of
+// this step or an earlier one, so every index derived from them stays inside
+// its buffer (the step's results are unspecified and reported).  Until the
+// condition has been reported, further steps sort nothing.
 // ---------------------------------------------------------------------------
-// After a scan wait gave up (status) the scatter and the rank pass leave
-// their outputs as they were: the step's results are unspecified and the
-// condition is reported.
-__global__ void k_scatter(int n, const int2* __restrict__ keySlot, const int* __restrict__ cellOffset,
-                          int* __restrict__ tmpIds, int* __restrict__ sortedHash, const int* __restrict__ skip,
-                          const unsigned int* __restrict__ status, const unsigned int* __restrict__ sortFlag) {
-    if ((skip && *skip) || (status && (*status & STATUS_DEVICE_WAIT)) || (sortFlag && !*sortFlag)) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int2 ks = keySlot[i];
-        int dst = __ldg(cellOffset + ks.x) + ks.y;
-        tmpIds[dst] = i;
-        sortedHash[dst] = ks.x;
-    }
-}
+constexpr int FRONT_THREADS = 512;
+constexpr int FRONT_WIDE = 1 << 19;
+constexpr int FRONT_WARPS = FRONT_THREADS / 32;
+// words of SortBuffers::front: barrier arrivals, blocks gone, a wait gave up, then the blocks' sums
+enum : int { FRONT_ARRIVED = 0, FRONT_GONE = 1, FRONT_FAILED = 2, FRONT_SUMS = 8 };
 
-void launch_scatter(int n, SortBuffers sb, cudaStream_t s, const unsigned int* status, const NeighbourLists* L) {
-    if (n <= 0) return;
-    k_scatter<<<stride_blocks(n), 256, 0, s>>>(n, sb.keySlot, sb.cellOffset, sb.tmpIds, sb.sortedHash, sb.skip,
-                                               status, sort_flag(L));
-}
+struct FrontArgs {
+    int n;
+    const float4* pos;
+    const float4* vel;
+    GridDev g;
+    SortBuffers sb;
+    float4* posS;
+    float4* velS;
+    unsigned int* status;
+    NeighbourLists L;
+    int lists;
+    int phases;
+    int waitLimit;
+};
 
-// ---------------------------------------------------------------------------
-// Stage 4: order each cell's members and gather the state into sorted order.
-// Two orders come out of one pass over the cell segment:
-//   by particle id   -> sortedIds, the reference's permutation (stable sort
-//                       by hash, particle_simulation.cu:2340), kept for the API;
-//   by (x, id)       -> workIds, the order the neighbour kernels use: a cell's
-//                       members sorted by x, so the lower and upper x-halves of
-//                       a cell are two contiguous ranges (halfOffset below).
-// Ranks count the smaller keys in the segment; x is compared through its
-// order-preserving integer image so the order is total (NaN included).
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned int ordered_bits(float x) {
     unsigned int u = __float_as_uint(x);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// The same pass records, per cell, where its upper x-half starts in the
-// working order (halfOffset[c] = first index with x >= the cell's mid-plane),
-// so a neighbour search can cut a row at half-cell granularity from a table.
-// With reused neighbour lists (`vl`) and no build in this step, the working
-// order is the one kept since the build (workIds): only the reference
-// permutation is ranked, and the state is gathered into the kept order.
-template <bool BATCH, bool REL>
-__global__ void k_rank_gather(int n, const int* __restrict__ sortedHash, const int* __restrict__ cellOffset,
-                              const int* __restrict__ tmpIds, const float4* __restrict__ pos,
-                              const float4* __restrict__ vel, GridDev g_, const SceneDev* __restrict__ scenes,
-                              int* __restrict__ sortedIds, int* __restrict__ workIds, int* __restrict__ halfOffset,
-                              float4* __restrict__ posS, float4* __restrict__ velS, const int* __restrict__ skip,
-                              const unsigned int* __restrict__ vl, int vlScenes, const int* __restrict__ slotScene,
-                              unsigned int* status) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || (skip && *skip) || (status && (*status & STATUS_DEVICE_WAIT))) return;
-    const int sc = BATCH && vl ? slotScene[k] : 0;  // the scene of sorted slot k
-    if (vl && !vl[VL_FLAGS * vlScenes + VL_SORT]) {
-        // no sort in this step: the state gathered into the kept order, with
-        // the hash pass's checks of each position
-        const int w = workIds[k];
-        const float4 p = __ldg(pos + w);
-        posS[k] = p;
-        velS[k] = __ldg(vel + w);
-        const GridDev& g = BATCH ? scenes[sc].g : g_;
+// Waits until every block of the grid has arrived `round` times.
+__device__ __forceinline__ bool grid_barrier(unsigned int* front, unsigned int round, int waitLimit, unsigned int* status) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> arrived(front[FRONT_ARRIVED]);
+        arrived.fetch_add(1u, cuda::memory_order_acq_rel);
+        const unsigned int all = round * gridDim.x;
+        int spins = 0;
+        ok = 1;
+        while (arrived.load(cuda::memory_order_acquire) < all || waitLimit < 0) {
+            if (++spins > waitLimit) {
+                ok = 0;
+                atomicOr(status, STATUS_DEVICE_WAIT);
+                atomicExch(front + FRONT_FAILED, 1u);
+                break;
+            }
+            __nanosleep(20);
+        }
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ int front_block_sum(int v, int* warps) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < FRONT_WARPS; w++) t += warps[w];
+    return t;
+}
+
+// What kind of step a scene takes: VL_BUILDS on request or when a particle
+// has moved farther than the skin allows since the last build (or the
+// displacement is not finite), VL_SEARCHES in place of a build that the last
+// step's own displacement would have outrun.
+__device__ __forceinline__ unsigned int list_kind(const NeighbourLists& L, const SceneDev* __restrict__ scenes, int k) {
+    const int S = L.numScenes;
+    const unsigned int* f = L.flags;
+    float lim2 = L.dispLimit2;
+    if (scenes) {
+        const float lim = 0.45f * L.skinFrac * scenes[k].ph.h;
+        lim2 = lim * lim;
+    }
+    if (f[VL_BUILD * S + k]) return VL_BUILDS;
+    const unsigned int last = f[VL_LAST * S + k];
+    if (!(__uint_as_float(f[VL_DISP * S + k]) <= lim2)) return last == VL_REUSES ? VL_BUILDS : VL_SEARCHES;
+    return last == VL_SEARCHES ? VL_BUILDS : VL_REUSES;
+}
+
+template <bool BATCH>
+__device__ __forceinline__ void front_gather(const FrontArgs& A) {
+    for (int k = blockIdx.x * FRONT_THREADS + threadIdx.x; k < A.n; k += gridDim.x * FRONT_THREADS) {
+        const int w = A.sb.workIds[k];
+        const float4 p = __ldg(A.pos + w), v = __ldg(A.vel + w);
+        A.posS[k] = p;
+        A.velS[k] = v;
+        const GridDev& g = BATCH ? A.sb.scenes[A.L.slotScene[k]].g : A.g;
         if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) {
-            atomicOr(status, STATUS_NON_FINITE);
+            atomicOr(A.status, STATUS_NON_FINITE);
         } else {
             bool outside = false;
             particle_hash(p, g, &outside);
-            if (outside) atomicOr(status, STATUS_OUT_OF_DOMAIN);
+            if (outside) atomicOr(A.status, STATUS_OUT_OF_DOMAIN);
         }
-        return;
     }
-    int c = sortedHash[k];
-    int s = __ldg(cellOffset + c), e = __ldg(cellOffset + c + 1);
-    int my = tmpIds[k];
-    if (vl && !vl[VL_BUILD_NOW * vlScenes + sc]) {
-        int rId = 0;
-        for (int t = s; t < e; t++) rId += __ldg(tmpIds + t) < my;
-        sortedIds[s + rId] = my;
-        const int w = workIds[k];
-        posS[k] = __ldg(pos + w);
-        velS[k] = __ldg(vel + w);
-        return;
-    }
-    float4 p = __ldg(pos + my);
-    const GridDev& g = BATCH ? scenes[__float_as_int(p.w)].g : g_;
-    unsigned int key = ordered_bits(p.x);
-    // the cell's mid-plane, in the frame its members' x is stored in
-    const float mid = REL ? 0.5f * g.spacing
-                          : g.origin[0] + ((float)((c - g.cellBase) % g.dim[0]) + 0.5f) * g.spacing;
-    int rId = 0, rX = 0, below = 0;
-    for (int t = s; t < e; t++) {
-        int o = __ldg(tmpIds + t);
-        float xo = __ldg(&pos[o].x);
-        unsigned int ko = ordered_bits(xo);
-        rId += o < my;
-        rX += (ko < key) || (ko == key && o < my);
-        below += xo < mid;
-    }
-    sortedIds[s + rId] = my;
-    workIds[s + rX] = my;
-    posS[s + rX] = p;
-    velS[s + rX] = __ldg(vel + my);
-    if (rX == 0) halfOffset[c] = s + below;
 }
 
-void launch_rank_gather(int n, SortBuffers sb, const float4* pos, const float4* vel, GridDev g, float4* posS,
-                        float4* velS, cudaStream_t s, const NeighbourLists* L, unsigned int* status) {
+// BATCH: the particle's scene (pos.w) supplies its grid, whose cells start at
+// that scene's cellBase in the concatenated cell space.  REL: the position is
+// cell-relative and the hash comes from its packed cell coordinates.
+template <bool BATCH, bool REL>
+__device__ __forceinline__ void front_hash(const FrontArgs& A) {
+    for (int i = blockIdx.x * FRONT_THREADS + threadIdx.x; i < A.n; i += gridDim.x * FRONT_THREADS) {
+        float4 p = A.pos[i];
+        const GridDev& g = BATCH ? A.sb.scenes[__float_as_int(p.w)].g : A.g;
+        bool outside = false;
+        const bool finite = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+        if (!finite) {
+            atomicOr(A.status, STATUS_NON_FINITE);
+            p = make_float4(g.origin[0], g.origin[1], g.origin[2], 0.f);
+        }
+        int h;
+        if (REL) {
+            const int3 c = finite ? rel_cell(p) : make_int3(0, 0, 0);
+            h = g.cellBase + g.dim[0] * (g.dim[1] * c.z + c.y) + c.x;
+        } else {
+            h = particle_hash(p, g, &outside);
+        }
+        if (outside) atomicOr(A.status, STATUS_OUT_OF_DOMAIN);
+        A.sb.keySlot[i] = make_int2(h, atomicAdd(A.sb.cnt + h, 1));
+    }
+}
+
+template <bool BATCH, bool REL>
+__device__ __forceinline__ void front_rank(const FrontArgs& A) {
+    // (plain loads: what earlier phases of this launch wrote)
+    for (int k = blockIdx.x * FRONT_THREADS + threadIdx.x; k < A.n; k += gridDim.x * FRONT_THREADS) {
+        const int c = A.sb.sortedHash[k];
+        const int s = A.sb.cellOffset[c], e = A.sb.cellOffset[c + 1];
+        const int my = A.sb.tmpIds[k];
+        if (A.lists && A.L.flags[VL_BUILD_NOW * A.L.numScenes + (BATCH ? A.L.slotScene[k] : 0)] == VL_REUSES) {
+            int rId = 0;
+            for (int t = s; t < e; t++) rId += A.sb.tmpIds[t] < my;
+            A.sb.sortedIds[s + rId] = my;
+            const int w = A.sb.workIds[k];
+            A.posS[k] = __ldg(A.pos + w);
+            A.velS[k] = __ldg(A.vel + w);
+            continue;
+        }
+        const float4 p = __ldg(A.pos + my);
+        const GridDev& g = BATCH ? A.sb.scenes[__float_as_int(p.w)].g : A.g;
+        const unsigned int key = ordered_bits(p.x);
+        // the cell's mid-plane, in the frame its members' x is stored in
+        const float mid = REL ? 0.5f * g.spacing
+                              : g.origin[0] + ((float)((c - g.cellBase) % g.dim[0]) + 0.5f) * g.spacing;
+        int rId = 0, rX = 0, below = 0;
+        for (int t = s; t < e; t++) {
+            const int o = A.sb.tmpIds[t];
+            const float xo = __ldg(&A.pos[o].x);
+            const unsigned int ko = ordered_bits(xo);
+            rId += o < my;
+            rX += (ko < key) || (ko == key && o < my);
+            below += xo < mid;
+        }
+        A.sb.sortedIds[s + rId] = my;
+        A.sb.workIds[s + rX] = my;
+        A.posS[s + rX] = p;
+        A.velS[s + rX] = __ldg(A.vel + my);
+        if (rX == 0) A.sb.halfOffset[c] = s + below;
+    }
+}
+
+template <bool BATCH, bool REL>
+__global__ void __launch_bounds__(FRONT_THREADS, 3) k_front(FrontArgs A) {
+    __shared__ int warps[FRONT_WARPS];
+    __shared__ int carry;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned int* front = A.sb.front;
+    if (A.sb.skip && *A.sb.skip) return;
+    bool ok = !(*(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT);
+    unsigned int* f = A.L.flags;
+    const int S = A.L.numScenes;
+    if (ok && A.lists) {
+        // The decision, or (a launch of later phases alone) what it was.  What
+        // it is taken from changes with the rank phase, when every block has
+        // decided (where nothing sorts, to what gives the same decision again).
+        bool sorts = false;
+        if (A.phases & FRONT_HASH) {
+            for (int k = t; k < S; k += FRONT_THREADS) {
+                const unsigned int kind = list_kind(A.L, A.sb.scenes, k);
+                sorts |= kind != VL_REUSES;
+                if (blockIdx.x == 0) f[VL_BUILD_NOW * S + k] = kind;
+            }
+            sorts = __syncthreads_or(sorts);
+            if (blockIdx.x == 0 && t == 0) {
+                f[VL_FLAGS * S + VL_SORT] = sorts ? 1u : 0u;
+                f[VL_FLAGS * S + VL_STALE] = sorts ? 0u : 1u;
+            }
+        } else {
+            sorts = f[VL_FLAGS * S + VL_SORT] != 0u;
+        }
+        if (!sorts) {
+            if (!(A.phases & FRONT_RANK)) return;
+            if (blockIdx.x == 0)
+                for (int k = t; k < S; k += FRONT_THREADS) f[VL_LAST * S + k] = VL_REUSES;
+            front_gather<BATCH>(A);
+            return;
+        }
+    }
+    unsigned int round = 0;
+    auto barrier = [&]() { ok = grid_barrier(front, ++round, A.waitLimit, A.status); };
+    if (ok && (A.phases & FRONT_HASH)) {
+        front_hash<BATCH, REL>(A);
+        if (A.phases & FRONT_SCAN) barrier();
+    }
+    // this block's stretch of cells, four at a time (the buffers are padded)
+    const long long total = ((long long)A.g.numCells + 4) & ~3ll;  // numCells + 1 counts
+    const long long per = ((total / 4 + gridDim.x - 1) / gridDim.x) * 4;
+    const long long c0 = per * blockIdx.x, c1 = min(c0 + per, total);
+    if (ok && (A.phases & FRONT_SUM)) {
+        int sum = 0;
+        for (long long c = c0 + 4 * t; c < c1; c += 4 * FRONT_THREADS) {
+            const int4 v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
+            sum += v.x + v.y + v.z + v.w;
+        }
+        sum = front_block_sum(sum, warps);
+        if (t == 0) front[FRONT_SUMS + blockIdx.x] = (unsigned int)sum;
+        barrier();
+    }
+    if (ok && (A.phases & FRONT_SCAN)) {
+        int before = 0;
+        for (int b = t; b < (int)blockIdx.x; b += FRONT_THREADS) before += (int)front[FRONT_SUMS + b];
+        before = front_block_sum(before, warps);
+        for (long long base = c0; base < c1; base += 4 * FRONT_THREADS) {
+            const long long c = base + 4 * t;
+            int4 v = make_int4(0, 0, 0, 0);
+            if (c < c1) {
+                v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
+                *reinterpret_cast<int4*>(A.sb.cnt + c) = make_int4(0, 0, 0, 0);
+            }
+            const int local = v.x + v.y + v.z + v.w;
+            int incl = local;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            __syncthreads();  // (the last use of `warps` and `carry`)
+            if (lane == 31) warps[warp] = incl;
+            __syncthreads();
+            int run = before + incl - local;
+            for (int w = 0; w < warp; w++) run += warps[w];
+            if (t == FRONT_THREADS - 1) carry = run + local;
+            if (c < c1) {
+                int4 o;
+                o.x = run;
+                o.y = o.x + v.x;
+                o.z = o.y + v.y;
+                o.w = o.z + v.z;
+                *reinterpret_cast<int4*>(A.sb.cellOffset + c) = o;
+                if (A.sb.halfOffset) *reinterpret_cast<int4*>(A.sb.halfOffset + c) = o;
+            }
+            __syncthreads();
+            before = carry;
+        }
+        if (A.phases & FRONT_SCATTER) barrier();
+    }
+    if (ok && (A.phases & FRONT_SCATTER)) {
+        for (int i = blockIdx.x * FRONT_THREADS + t; i < A.n; i += gridDim.x * FRONT_THREADS) {
+            const int2 ks = A.sb.keySlot[i];
+            const int dst = A.sb.cellOffset[ks.x] + ks.y;
+            A.sb.tmpIds[dst] = i;
+            A.sb.sortedHash[dst] = ks.x;
+        }
+        if (A.phases & FRONT_RANK) barrier();
+    }
+    if (ok && (A.phases & FRONT_RANK)) {
+        if (A.lists && blockIdx.x == 0) {
+            for (int k = t; k < S; k += FRONT_THREADS) {
+                const unsigned int kind = f[VL_BUILD_NOW * S + k];
+                f[VL_LAST * S + k] = kind;
+                f[VL_BUILD * S + k] = 0u;
+                if (kind != VL_REUSES) {
+                    f[VL_DISP * S + k] = 0u;
+                    if (kind == VL_BUILDS) f[VL_COUNT * S + k] += 1u;
+                }
+            }
+        }
+        front_rank<BATCH, REL>(A);
+    }
+    // the last block to leave readies the words for the next launch
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        carry = atomicAdd(front + FRONT_GONE, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!carry) return;
+    __threadfence();
+    if (*(volatile unsigned int*)(front + FRONT_FAILED)) {
+        for (long long c = t; c < total; c += FRONT_THREADS) A.sb.cnt[c] = 0;
+        if (A.lists)
+            for (int k = t; k < S; k += FRONT_THREADS) f[VL_BUILD * S + k] = 1u;
+    }
+    __syncthreads();
+    if (t < FRONT_SUMS) front[t] = 0u;
+}
+
+// `perSm` blocks of k_front an SM, as far as the current device holds them at once.
+template <bool BATCH, bool REL>
+static int front_resident(int perSm) {
+    static std::atomic<int> known[64];  // blocks an SM times 4096, plus SMs
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int k = dev < 64 ? known[dev].load() : 0;
+    if (k == 0) {
+        int fit = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_front<BATCH, REL>, FRONT_THREADS, 0) != cudaSuccess ||
+            fit < 1)
+            fit = 1;
+        k = fit * 4096 + std::min(device_sms(), 4095);
+        if (dev < 64) known[dev].store(k);
+    }
+    return std::min(std::min(perSm, k / 4096) * (k % 4096), FRONT_MAX_BLOCKS);
+}
+
+template <bool BATCH, bool REL>
+static void front_launch(FrontArgs A, cudaStream_t s) {
+    // one particle a thread and sixteen cells, as far as the blocks may be
+    const long long want = std::max(((long long)A.n + FRONT_THREADS - 1) / FRONT_THREADS,
+                                    ((long long)A.g.numCells + 16 * FRONT_THREADS) / (16 * FRONT_THREADS));
+    const int most = front_resident<BATCH, REL>(A.n > FRONT_WIDE ? 2 : 1);
+    const int grid = (int)std::max(1ll, std::min(want, (long long)most));
+    void* args[] = {&A};
+    cudaLaunchCooperativeKernel((const void*)k_front<BATCH, REL>, dim3(grid), dim3(FRONT_THREADS), args, 0, s);
+}
+
+void launch_front(int n, const float4* pos, const float4* vel, GridDev g, SortBuffers sb, float4* posS, float4* velS,
+                  unsigned int* status, cudaStream_t s, const NeighbourLists* L, int phases) {
     if (n <= 0) return;
-    const int grid = (n + 255) / 256;
-    const unsigned int* vl = L ? L->flags : nullptr;
-    const int vs = L ? L->numScenes : 1;
-    const int* ss = L ? L->slotScene : nullptr;
-    if (sb.scenes)
-        k_rank_gather<true, false><<<grid, 256, 0, s>>>(n, sb.sortedHash, sb.cellOffset, sb.tmpIds, pos, vel, g,
-                                                        sb.scenes, sb.sortedIds, sb.workIds, sb.halfOffset, posS,
-                                                        velS, sb.skip, vl, vs, ss, status);
-    else if (g.rel)
-        k_rank_gather<false, true><<<grid, 256, 0, s>>>(n, sb.sortedHash, sb.cellOffset, sb.tmpIds, pos, vel, g,
-                                                        nullptr, sb.sortedIds, sb.workIds, sb.halfOffset, posS, velS,
-                                                        sb.skip, nullptr, 1, nullptr, status);
-    else
-        k_rank_gather<false, false><<<grid, 256, 0, s>>>(n, sb.sortedHash, sb.cellOffset, sb.tmpIds, pos, vel, g,
-                                                         nullptr, sb.sortedIds, sb.workIds, sb.halfOffset, posS,
-                                                         velS, sb.skip, vl, vs, nullptr, status);
+    FrontArgs A{n, pos, vel, g, sb, posS, velS, status, L ? *L : NeighbourLists{}, L ? 1 : 0, phases, scan_wait_limit()};
+    if (sb.scenes) front_launch<true, false>(A, s);
+    else if (g.rel) front_launch<false, true>(A, s);
+    else front_launch<false, false>(A, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -565,9 +706,8 @@ void launch_rebuild_tables(int n, const float4* posS, const int* workIds, const 
     sb.skip = nullptr;
     sb.halfOffset = nullptr;  // stays the working order's
     k_unsort_positions<<<(n + 255) / 256, 256, 0, s>>>(n, posS, workIds, slotScene, scratch);
-    launch_hash_count(n, scratch, g, sb, status, s, nullptr);
-    launch_cell_scan(g.numCells, sb, status, s, nullptr);
-    launch_scatter(n, sb, s, status, nullptr);
+    launch_front(n, scratch, nullptr, g, sb, nullptr, nullptr, status, s, nullptr,
+                 FRONT_HASH | FRONT_SUM | FRONT_SCAN | FRONT_SCATTER);
     k_rank_ids<<<(n + 255) / 256, 256, 0, s>>>(n, sb.sortedHash, sb.cellOffset, sb.tmpIds, sb.sortedIds);
 }
 

@@ -155,17 +155,13 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
 // within h), and only the set bits are appended: an append costs as much as a
 // test and a quarter of the candidates pass.
 // ---------------------------------------------------------------------------
-// BATCH: the slot's scene supplies grid, constants, maps, R and the scene's
-// own decision.
+// BATCH: the slot's scene supplies grid, constants, maps and R.
 template <bool KAHAN, bool BATCH>
-__device__ __forceinline__ void density_build_one(int i, int n, float4* posS, float4* velS, const RowTables& T,
+__device__ __forceinline__ void density_build_one(int i, int n, bool lists, int scene, float4* posS, float4* velS,
+                                                  const RowTables& T,
                                                   const GridDev& g_, const PhysDev& ph_, const MapDev& map_,
                                                   float4* __restrict__ rho4S, const NeighbourLists& L,
                                                   const RowMasks& M) {
-    const int scene = BATCH ? L.slotScene[i] : 0;
-    const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
-    if (kind == VL_REUSES) return;
-    const bool lists = kind == VL_BUILDS;
     const float4 xi = posS[i];
     const SceneDev* S = BATCH ? T.scenes + scene : nullptr;
     const GridDev& g = BATCH ? S->g : g_;
@@ -273,32 +269,28 @@ __device__ __forceinline__ void density_build_one(int i, int n, float4* posS, fl
     velS[i].w = inv;
 }
 
-// (A grid of one wave striding over the particles would make the early
-// return cheaper, but the build itself ran 15 % slower that way.)
-template <bool KAHAN, bool BATCH>
-__global__ void __launch_bounds__(256, 4)
-k_density_build(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
-    if (!BATCH && !L.flags[VL_BUILD_NOW]) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        density_build_one<KAHAN, BATCH>(i, n, posS, velS, T, g, ph, map, rho4S, L, M);
-}
-
+constexpr int DENSITY_LIST_BLOCKS = 4;
+// The density stage of a list step: the build form above where the scene's
+// step does not reuse its lists.
 // List form: the candidates within R, four at a time; each group's terms are
 // summed in plain FP32 (as a row's few terms are) and the group sums are
 // added with compensation.  The next group's slots are loaded before the
 // current group's positions are used.
 template <bool KAHAN, bool BATCH>
-__global__ void __launch_bounds__(256, 6)
-k_density_lists(int n, float4* posS, float4* velS, PhysDev ph_, MapDev map_, float4* __restrict__ rho4S,
-                NeighbourLists L, const SceneDev* __restrict__ scenes) {
+__global__ void __launch_bounds__(256, DENSITY_LIST_BLOCKS)
+k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph_, MapDev map_,
+                float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int scene = BATCH ? L.slotScene[i] : 0;
-    if (L.flags[VL_BUILD_NOW * L.numScenes + scene]) return;
+    const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
+    if (kind != VL_REUSES) {
+        density_build_one<KAHAN, BATCH>(i, n, kind == VL_BUILDS, scene, posS, velS, T, g, ph_, map_, rho4S, L, M);
+        return;
+    }
     const float4 xi = posS[i];
-    const PhysDev& ph = BATCH ? scenes[scene].ph : ph_;
-    const MapDev& map = BATCH ? scenes[scene].map : map_;
+    const PhysDev& ph = BATCH ? T.scenes[scene].ph : ph_;
+    const MapDev& map = BATCH ? T.scenes[scene].map : map_;
     const float h2 = ph.h2;
     const unsigned int groups = L.groups[i];
     float sum = 0.f, comp = 0.f;
@@ -1468,34 +1460,18 @@ void launch_list_displacement(int n, const float4* pos, const int* workIds, cons
 }
 
 void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
-                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg, bool build,
-                          bool reuse, cudaStream_t s) {
+                          float4* rho4S, const NeighbourLists& L, RowMasks M, const StepConfig& cfg, cudaStream_t s) {
     if (n <= 0) return;
     const int bs = cfg.densityBlock > 0 ? cfg.densityBlock : 128;
     const int grid = (n + bs - 1) / bs;
-    const bool batch = T.scenes != nullptr;
-#define SPH_DENSITY_BUILD(K, B) k_density_build<K, B><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L, M)
-#define SPH_DENSITY_LISTS(K, B) \
-    k_density_lists<K, B><<<grid, bs, 0, s>>>(n, posS, velS, ph, map, rho4S, L, T.scenes)
-    if (build) {
-        if (cfg.kahan) {
-            if (batch) SPH_DENSITY_BUILD(true, true);
-            else SPH_DENSITY_BUILD(true, false);
-        } else {
-            if (batch) SPH_DENSITY_BUILD(false, true);
-            else SPH_DENSITY_BUILD(false, false);
-        }
+#define SPH_DENSITY_LISTS(K, B) k_density_lists<K, B><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L, M)
+    if (cfg.kahan) {
+        if (T.scenes) SPH_DENSITY_LISTS(true, true);
+        else SPH_DENSITY_LISTS(true, false);
+    } else {
+        if (T.scenes) SPH_DENSITY_LISTS(false, true);
+        else SPH_DENSITY_LISTS(false, false);
     }
-    if (reuse) {
-        if (cfg.kahan) {
-            if (batch) SPH_DENSITY_LISTS(true, true);
-            else SPH_DENSITY_LISTS(true, false);
-        } else {
-            if (batch) SPH_DENSITY_LISTS(false, true);
-            else SPH_DENSITY_LISTS(false, false);
-        }
-    }
-#undef SPH_DENSITY_BUILD
 #undef SPH_DENSITY_LISTS
 }
 

@@ -551,7 +551,9 @@ sph_status sph_autotune(sph_handle h, int reps, sph_tuning* chosen);
  * 2 scatter, 3 rank_gather, 4 density, 5 force_integrate -- every plain and
  * two-scale step -- then, in two-scale steps only, 6 ts_children (states,
  * split lists, children, projection), 7 sub_sort, 8 sub_density, 9 sub_force.
- * An interval holds its stage's launches and the gaps between them. */
+ * An interval holds its stage's launches and the gaps between them (stages 0
+ * to 3 are phases of one launch in an untimed step, launches of their own in
+ * a timed one). */
 sph_status sph_set_stage_timing(sph_handle h, int enable);
 sph_status sph_stage_times(sph_handle h, float* ms, int* counts, int capacity, int* numStages);
 const char* sph_stage_name(int stage);
