@@ -629,23 +629,16 @@ sph_status sph_boundary_maps(const sph_boundary_desc* desc, float* distance, flo
     sph_status st = check_desc(desc, dims);
     if (st) return st;
     size_t total = (size_t)dims[0] * dims[1] * dims[2];
-    float *d = nullptr, *r = nullptr, *v = nullptr;
-    SPH_CUDA(dalloc(&d, total));
-    cudaError_t e1 = dalloc(&r, total), e2 = dalloc(&v, total);
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        cudaFree(d);
-        if (r) cudaFree(r);
-        if (v) cudaFree(v);
-        SPH_FAIL(SPH_ERR_OUT_OF_MEMORY, "boundary map allocation failed");
-    }
+    // the three maps in one allocation (each allocation and release costs ~50 us)
+    float* d = nullptr;
+    if (dalloc(&d, 3 * total) != cudaSuccess) SPH_FAIL(SPH_ERR_OUT_OF_MEMORY, "boundary map allocation failed");
+    float *r = d + total, *v = r + total;
     cudaError_t e = launch_build_maps(*desc, dims, d, r, v, nullptr, 0);
     if (e == cudaSuccess && distance) e = cudaMemcpy(distance, d, total * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && density) e = cudaMemcpy(density, r, total * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && viscosity) e = cudaMemcpy(viscosity, v, total * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     cudaFree(d);
-    cudaFree(r);
-    cudaFree(v);
     SPH_CUDA(e);
     return SPH_OK;
 }

@@ -15,9 +15,12 @@
 // for a 128^3 map.  The lattice's ghosts are now found once, as one bit a
 // lattice point, and the nodes walk the set bits; a distance is taken in FP64
 // only where an FP32 one with a bound on its error cannot decide; the
-// coefficients are formed on the host.  22.8 -> 0.52 ms for that map (sphere
-// and cone, 125,000 of 2.1 M nodes in the band; 10 us of it the lattice).
+// coefficients are formed on the host; the band's nodes are listed, so that the
+// sums fill their warps.  22.8 -> 0.20 ms for that map (sphere and cone;
+// lattice 9 us, distances 69, sums of the band's nodes 125).
 #include <math.h>
+
+#include <algorithm>
 
 #include "sph_internal.h"
 
@@ -39,6 +42,7 @@ struct MapArgs {
     unsigned int rowWords;
     float densityCoeff;      // evaluateDensityKernel's and evaluateViscosityKernel's coefficients
     double viscosityCoeff;
+    float viscosityHi, viscosityLo;  // the same as a sum of two floats; hi 0: out of their range
     // SPH_SHAPE_MESH solids: the signed distance grid of shape slot i
     const float* grid[8];
     float gridOrigin[8][3];
@@ -184,7 +188,12 @@ __device__ float eval_density_kernel(const MapArgs& A, float sqDist) {
 __device__ float eval_viscosity_kernel(const MapArgs& A, float sqDist) {
     float dist = sqrtf(sqDist);
     if (dist > A.h) return 0.0f;
-    return (float)(A.viscosityCoeff * (A.h - dist));
+    const float x = A.h - dist;
+    if (A.viscosityHi == 0.0f) return (float)(A.viscosityCoeff * x);
+    // the FP64 product rounded to FP32, from FP32 operations (the FP64 pipe and
+    // its conversions held the sums: 315 -> 125 us for a 128^3 map)
+    const float p = A.viscosityHi * x;
+    return p + __fmaf_rn(A.viscosityLo, x, __fmaf_rn(A.viscosityHi, x, -p));
 }
 
 __device__ void node_pos(const MapArgs& A, int i, int j, int k, float* p) {
@@ -215,69 +224,117 @@ __global__ void k_ghost_bits(MapArgs A, unsigned int* __restrict__ bits, size_t 
     if ((threadIdx.x & 31u) == 0u) bits[w] = m;
 }
 
-__global__ void k_build_maps(MapArgs A, float* dist, float* dens, float* visc, float4* map4) {
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t total = (size_t)A.dims[0] * A.dims[1] * A.dims[2];
-    if (n >= total) return;
-    int i = (int)(n % A.dims[0]);
-    int j = (int)((n / A.dims[0]) % A.dims[1]);
-    int k = (int)(n / ((size_t)A.dims[0] * A.dims[1]));
-    float np[3];
-    node_pos(A, i, j, k, np);
-    float margin;
-    const float est = solid_estimate(A, np, margin);
-    float outD = -A.restDistance, outRho = 0.0f, outVis = 0.0f;
-    // a node certainly beyond the band needs no distance
-    float d = fabsf(est) - margin > A.h ? A.h : -solid_distance(A, np);
-    if (fabsf(d) < A.h) {
-        if (fabsf(d) > A.restDistance) d = d / fabsf(d) * A.restDistance;
-        outD = d;
-        // ghost lattice points that can lie within h of this node
-        int lo[3], hi[3];
-        for (int a = 0; a < 3; a++) {
-            float f0 = floorf((np[a] - A.h - A.latStart[a]) / A.ps) - 1.0f;
-            float f1 = floorf((np[a] + A.h - A.latStart[a]) / A.ps) + 1.0f;
-            f0 = fmaxf(f0, 0.0f);
-            f1 = fminf(f1, (float)A.latMax[a]);
-            lo[a] = (int)f0;
-            hi[a] = (int)f1;
-        }
-        auto add = [&](int ii, float gy, float gz) {
-            const float dx = A.latStart[0] + (float)ii * A.ps - np[0], dy = gy - np[1], dz = gz - np[2];
-            const float sq = dx * dx + dy * dy + dz * dz;
-            outRho += eval_density_kernel(A, sq);
-            outVis += eval_viscosity_kernel(A, sq);
-        };
-        for (int kk = lo[2]; kk <= hi[2]; kk++)
-            for (int jj = lo[1]; jj <= hi[1]; jj++) {
-                const float gy = A.latStart[1] + (float)jj * A.ps, gz = A.latStart[2] + (float)kk * A.ps;
-                if (!A.ghosts) {
-                    for (int ii = lo[0]; ii <= hi[0]; ii++) {
-                        const float g[3] = {A.latStart[0] + (float)ii * A.ps, gy, gz};
-                        if (is_ghost(A, g)) add(ii, gy, gz);
-                    }
-                    continue;
+// The density and viscosity of node n in the band (position np).
+__device__ void splat_node(const MapArgs& A, const float* np, float& outRho, float& outVis) {
+    // ghost lattice points that can lie within h of this node
+    int lo[3], hi[3];
+    for (int a = 0; a < 3; a++) {
+        float f0 = floorf((np[a] - A.h - A.latStart[a]) / A.ps) - 1.0f;
+        float f1 = floorf((np[a] + A.h - A.latStart[a]) / A.ps) + 1.0f;
+        f0 = fmaxf(f0, 0.0f);
+        f1 = fminf(f1, (float)A.latMax[a]);
+        lo[a] = (int)f0;
+        hi[a] = (int)f1;
+    }
+    outRho = outVis = 0.0f;
+    auto add = [&](int ii, float gy, float gz) {
+        const float dx = A.latStart[0] + (float)ii * A.ps - np[0], dy = gy - np[1], dz = gz - np[2];
+        const float sq = dx * dx + dy * dy + dz * dz;
+        outRho += eval_density_kernel(A, sq);
+        outVis += eval_viscosity_kernel(A, sq);
+    };
+    for (int kk = lo[2]; kk <= hi[2]; kk++)
+        for (int jj = lo[1]; jj <= hi[1]; jj++) {
+            const float gy = A.latStart[1] + (float)jj * A.ps, gz = A.latStart[2] + (float)kk * A.ps;
+            if (!A.ghosts) {
+                for (int ii = lo[0]; ii <= hi[0]; ii++) {
+                    const float g[3] = {A.latStart[0] + (float)ii * A.ps, gy, gz};
+                    if (is_ghost(A, g)) add(ii, gy, gz);
                 }
-                const unsigned int* row =
-                    A.ghosts + ((size_t)kk * (A.latMax[1] + 1u) + (size_t)jj) * A.rowWords;
-                for (int w = lo[0] >> 5; w <= hi[0] >> 5; w++) {
-                    unsigned int m = __ldg(row + w);
-                    if (w == lo[0] >> 5) m &= 0xffffffffu << (lo[0] & 31);
-                    if (w == hi[0] >> 5) m &= 0xffffffffu >> (31 - (hi[0] & 31));
-                    while (m) {
-                        const int b = __ffs(m) - 1;
-                        m &= m - 1u;
-                        add(32 * w + b, gy, gz);
-                    }
+                continue;
+            }
+            const unsigned int* row = A.ghosts + ((size_t)kk * (A.latMax[1] + 1u) + (size_t)jj) * A.rowWords;
+            for (int w = lo[0] >> 5; w <= hi[0] >> 5; w++) {
+                unsigned int m = __ldg(row + w);
+                if (w == lo[0] >> 5) m &= 0xffffffffu << (lo[0] & 31);
+                if (w == hi[0] >> 5) m &= 0xffffffffu >> (31 - (hi[0] & 31));
+                while (m) {
+                    const int b = __ffs(m) - 1;
+                    m &= m - 1u;
+                    add(32 * w + b, gy, gz);
                 }
             }
-        outRho *= A.mass;
-        outVis *= A.viscosity * A.mass / A.restDensity;
+        }
+    outRho *= A.mass;
+    outVis *= A.viscosity * A.mass / A.restDensity;
+}
+
+struct MapOut {
+    float *dist, *dens, *visc;
+    float4* map4;
+    __device__ void store(size_t n, float d, float rho, float vis) const {
+        if (dist) dist[n] = d;
+        if (dens) dens[n] = rho;
+        if (visc) visc[n] = vis;
+        if (map4) map4[n] = make_float4(d, rho, vis, 0.0f);
     }
-    if (dist) dist[n] = outD;
-    if (dens) dens[n] = outRho;
-    if (visc) visc[n] = outVis;
-    if (map4) map4[n] = make_float4(outD, outRho, outVis, 0.0f);
+};
+
+__device__ void node_of(const MapArgs& A, size_t n, float* np) {
+    const int i = (int)(n % A.dims[0]);
+    const int j = (int)((n / A.dims[0]) % A.dims[1]);
+    const int k = (int)(n / ((size_t)A.dims[0] * A.dims[1]));
+    node_pos(A, i, j, k, np);
+}
+
+// Every node's distance.  The nodes in the band (one in twenty, scattered
+// over the warps) are listed for k_splat_band, which fills its warps with
+// them; without room for the list each thread takes its own node's sums.
+__global__ void k_build_maps(MapArgs A, MapOut out, unsigned int* band, unsigned int* bandCount) {
+    const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = n < (size_t)A.dims[0] * A.dims[1] * A.dims[2];
+    float np[3] = {0.0f, 0.0f, 0.0f};
+    float outD = -A.restDistance, outRho = 0.0f, outVis = 0.0f;
+    bool inBand = false;
+    if (valid) {
+        node_of(A, n, np);
+        float margin;
+        const float est = solid_estimate(A, np, margin);
+        // a node certainly beyond the band needs no distance
+        float d = fabsf(est) - margin > A.h ? A.h : -solid_distance(A, np);
+        inBand = fabsf(d) < A.h;
+        if (inBand) {
+            if (fabsf(d) > A.restDistance) d = d / fabsf(d) * A.restDistance;
+            outD = d;
+        }
+    }
+    if (band) {
+        const unsigned int peers = __ballot_sync(0xffffffffu, inBand), lane = threadIdx.x & 31u;
+        unsigned int at = 0u;
+        if (lane == 0u && peers) at = atomicAdd(bandCount, (unsigned int)__popc(peers));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(peers & ((1u << lane) - 1u));
+        if (inBand) band[at] = (unsigned int)n;
+    } else if (inBand) {
+        splat_node(A, np, outRho, outVis);
+    }
+    if (valid) out.store(n, outD, outRho, outVis);
+}
+
+__global__ void __launch_bounds__(128) k_splat_band(MapArgs A, MapOut out, const unsigned int* __restrict__ band,
+                                                    const unsigned int* __restrict__ bandCount) {
+    const unsigned int count = *bandCount;
+    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+        const size_t n = band[k];
+        float np[3], rho, vis;
+        node_of(A, n, np);
+        splat_node(A, np, rho, vis);
+        if (out.dens) out.dens[n] = rho;
+        if (out.visc) out.visc[n] = vis;
+        if (out.map4) {
+            out.map4[n].y = rho;
+            out.map4[n].z = vis;
+        }
+    }
 }
 
 // Lattices of up to 2^26 words (256 MB of bits) have their ghosts found once.
@@ -330,6 +387,10 @@ cudaError_t launch_build_maps(const sph_boundary_desc& D, const unsigned int dim
     const float h = A.h;
     A.densityCoeff = (float)(315.0f / (64.0f * 3.14159265358979323846 * h * h * h * h * h * h * h * h * h));
     A.viscosityCoeff = 45.0f / (3.14159265358979323846 * h * h * h * h * h * h);
+    if (A.viscosityCoeff > 1e-20 && A.viscosityCoeff < 1e20) {
+        A.viscosityHi = (float)A.viscosityCoeff;
+        A.viscosityLo = (float)(A.viscosityCoeff - (double)A.viscosityHi);
+    }
     // grid solids: device copies of their distances for the build
     float* devGrid[8] = {};
     cudaError_t e = cudaSuccess;
@@ -346,27 +407,35 @@ cudaError_t launch_build_maps(const sph_boundary_desc& D, const unsigned int dim
             A.gridDims[i][a] = G.dims[a];
         }
     }
-    unsigned int* bits = nullptr;
+    // scratch of the build: the band's count and node list, the lattice's bits
     A.rowWords = A.latMax[0] / 32u + 1u;
     const double wanted = (double)A.rowWords * ((double)A.latMax[1] + 1.0) * ((double)A.latMax[2] + 1.0);
     const size_t words = wanted <= GHOST_WORDS_MAX ? (size_t)wanted : 0;
-    if (e == cudaSuccess && words) {
-        if (cudaMallocAsync((void**)&bits, sizeof(unsigned int) * words, s) != cudaSuccess) {
-            cudaGetLastError();  // no room: the nodes test the lattice themselves
-            bits = nullptr;
-        }
+    const MapOut out{dist, dens, visc, map4};
+    unsigned int* scratch = nullptr;
+    if (e == cudaSuccess && cudaMallocAsync((void**)&scratch, sizeof(unsigned int) * (4 + total + words), s) != cudaSuccess) {
+        cudaGetLastError();  // no room: the nodes test the lattice and take their sums themselves
+        scratch = nullptr;
     }
-    if (bits) {
+    unsigned int *count = scratch, *band = scratch ? scratch + 4 : nullptr;
+    if (scratch) e = cudaMemsetAsync(count, 0, sizeof(unsigned int), s);
+    if (scratch && words && e == cudaSuccess) {
+        unsigned int* bits = band + total;
         k_ghost_bits<<<(unsigned int)((words + 3) / 4), 128, 0, s>>>(A, bits, words);
         e = cudaGetLastError();
         A.ghosts = bits;
     }
     if (e == cudaSuccess) {
-        k_build_maps<<<(unsigned int)((total + 127) / 128), 128, 0, s>>>(A, dist, dens, visc, map4);
+        k_build_maps<<<(unsigned int)((total + 127) / 128), 128, 0, s>>>(A, out, band, count);
         e = cudaGetLastError();
     }
-    if (bits) {
-        const cudaError_t f = cudaFreeAsync(bits, s);
+    if (band && e == cudaSuccess) {
+        const size_t full = (size_t)device_sms() * 12;
+        k_splat_band<<<(unsigned int)std::min((total + 127) / 128, full), 128, 0, s>>>(A, out, band, count);
+        e = cudaGetLastError();
+    }
+    if (scratch) {
+        const cudaError_t f = cudaFreeAsync(scratch, s);
         if (e == cudaSuccess) e = f;
     }
     bool any = false;
