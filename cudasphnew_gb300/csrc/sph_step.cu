@@ -1115,9 +1115,12 @@ constexpr int L_BAR = L_NORM + 4 * mlp::NNORM;  // MMA barrier, TMEM slot, weigh
 constexpr int L_SMEM = L_BAR + 32;
 constexpr int L_TMEM = 128;                   // 4 blocks x 128 = 512 columns
 constexpr int L_THREADS = 256;
-// Resident blocks per SM: four (64 registers, a few spilled) when the grid
-// fills the GPU several times over, the pair loop being latency bound; three
-// (80 registers, no spills) for small grids, where per-thread latency counts.
+// Resident blocks per SM.  Over the lists three (80 registers): a group's
+// gathers are in flight together, and four blocks' 64 registers spill them
+// (524,288 particles 221 us a step with three, 249 with four, 235 with two;
+// 60,000: 50, 57, 48).  With the per-step search four when the grid fills the
+// GPU several times over, the pair loop being latency bound; three for small
+// grids, where per-thread latency counts.
 constexpr int L_BLOCKS_MAX = 4;
 static_assert(L_X % 1024 == 0 && L_BIAS % 16 == 0 && L_NORM % 16 == 0 && L_BAR % 8 == 0, "layout");
 static_assert(L_BLOCKS_MAX * (L_SMEM + 1024) <= 227 * 1024 && L_BLOCKS_MAX * L_TMEM <= 512,
@@ -1400,7 +1403,7 @@ static void force_learned_dispatch(const ForceArgs& F, MlpDev m, unsigned int* s
                                    cudaStream_t s) {
     const int sms = device_sms();
     const long long blocks = (F.n + L_THREADS - 1) / L_THREADS;
-    if (blocks >= 2LL * L_BLOCKS_MAX * sms)
+    if (!LISTS && blocks >= 2LL * L_BLOCKS_MAX * sms)
         force_learned_launch<KAHAN, TENSION, L_BLOCKS_MAX, LISTS>(F, m, status, L, s);
     else
         force_learned_launch<KAHAN, TENSION, 3, LISTS>(F, m, status, L, s);
