@@ -196,10 +196,10 @@ void free_all(sph_sim* s) {
         if (s->upLand[k]) cudaFree(s->upLand[k]);
         if (s->upReady[k]) cudaEventDestroy(s->upReady[k]);
         if (s->upFree[k]) cudaEventDestroy(s->upFree[k]);
+        if (s->downStage[k]) cudaFree(s->downStage[k]);
+        if (s->downReady[k]) cudaEventDestroy(s->downReady[k]);
+        if (s->downFree[k]) cudaEventDestroy(s->downFree[k]);
     }
-    if (s->downStage) cudaFree(s->downStage);
-    if (s->downReady) cudaEventDestroy(s->downReady);
-    if (s->downFree) cudaEventDestroy(s->downFree);
     if (s->ownStream) cudaStreamDestroy(s->ownStream);
 }
 
@@ -896,6 +896,17 @@ sph_status read_two_scale(sph_sim* s, int field, void* dst, size_t bytes) {
         SPH_CUDA(cudaStreamSynchronize(q));
         return SPH_OK;
     }
+    if (field == SPH_FIELD_SUB_VERTEX_DATA) {
+        // page-locked memory takes the positions from the kernel itself, over the
+        // host link (as read_field; 25 MB in 140 us, 300 through a device buffer
+        // allocated for the call)
+        if (float* direct = static_cast<float*>(host_device_ptr(dst))) {
+            launch_pack_aos(s->ts.subPos, (int)(8 * n), direct, 3, 0, q);
+            SPH_CUDA(cudaGetLastError());
+            SPH_CUDA(cudaStreamSynchronize(q));
+            return SPH_OK;
+        }
+    }
     float* tmp = nullptr;
     SPH_CUDA(cudaMalloc((void**)&tmp, need));
     if (field == SPH_FIELD_SUB_VERTEX_DATA) launch_pack_aos(s->ts.subPos, (int)(8 * n), tmp, 3, 0, q);
@@ -929,15 +940,15 @@ static cudaError_t ensure_side_streams(sph_sim* s) {
     if (s->upStream) return cudaSuccess;
     const size_t n3 = 3 * (size_t)s->n;
     cudaStream_t up = nullptr, down = nullptr;
-    float *land[2] = {nullptr, nullptr}, *stage = nullptr;
-    cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    float *land[2] = {nullptr, nullptr}, *stage[2] = {nullptr, nullptr};
+    cudaEvent_t ev[8] = {};
     cudaError_t e = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&down, cudaStreamNonBlocking);
     for (int k = 0; k < 2 && e == cudaSuccess; k++) e = dalloc(&land[k], n3);
-    if (e == cudaSuccess) e = dalloc(&stage, n3);
-    for (int k = 0; k < 6 && e == cudaSuccess; k++) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+    for (int k = 0; k < 2 && e == cudaSuccess; k++) e = dalloc(&stage[k], n3);
+    for (int k = 0; k < 8 && e == cudaSuccess; k++) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
     if (e != cudaSuccess) {
-        for (float* p : {land[0], land[1], stage})
+        for (float* p : {land[0], land[1], stage[0], stage[1]})
             if (p) cudaFree(p);
         for (cudaEvent_t x : ev)
             if (x) cudaEventDestroy(x);
@@ -951,10 +962,10 @@ static cudaError_t ensure_side_streams(sph_sim* s) {
         s->upLand[k] = land[k];
         s->upReady[k] = ev[k];
         s->upFree[k] = ev[2 + k];
+        s->downStage[k] = stage[k];
+        s->downReady[k] = ev[4 + k];
+        s->downFree[k] = ev[6 + k];
     }
-    s->downStage = stage;
-    s->downReady = ev[4];
-    s->downFree = ev[5];
     return cudaSuccess;
 }
 
@@ -986,8 +997,9 @@ static sph_status read_field(sph_sim* s, int field, void* dst, size_t bytes, boo
         // packed on the handle's stream into a buffer of its own, copied to
         // the host by DMA on the side stream: the next step need not wait
         SPH_CUDA(ensure_side_streams(s));
-        SPH_CUDA(cudaStreamWaitEvent(q, s->downFree, 0));
-        out = s->downStage;
+        s->downNext ^= 1;
+        SPH_CUDA(cudaStreamWaitEvent(q, s->downFree[s->downNext], 0));
+        out = s->downStage[s->downNext];
     }
     switch (field) {
         case SPH_FIELD_VERTEX_DATA:
@@ -1017,10 +1029,11 @@ static sph_status read_field(sph_sim* s, int field, void* dst, size_t bytes, boo
     }
     SPH_CUDA(cudaGetLastError());
     if (!wait) {
-        SPH_CUDA(cudaEventRecord(s->downReady, q));
-        SPH_CUDA(cudaStreamWaitEvent(s->downStream, s->downReady, 0));
-        SPH_CUDA(cudaMemcpyAsync(dst, s->downStage, need, cudaMemcpyDeviceToHost, s->downStream));
-        SPH_CUDA(cudaEventRecord(s->downFree, s->downStream));
+        const int k = s->downNext;
+        SPH_CUDA(cudaEventRecord(s->downReady[k], q));
+        SPH_CUDA(cudaStreamWaitEvent(s->downStream, s->downReady[k], 0));
+        SPH_CUDA(cudaMemcpyAsync(dst, s->downStage[k], need, cudaMemcpyDeviceToHost, s->downStream));
+        SPH_CUDA(cudaEventRecord(s->downFree[k], s->downStream));
         return SPH_OK;
     }
     if (!direct) SPH_CUDA(cudaMemcpyAsync(dst, s->staging, need, cudaMemcpyDeviceToHost, q));
@@ -1061,7 +1074,7 @@ sph_status sph_write(sph_handle s, int field, const void* src, size_t bytes) {
     if (!s || !src) SPH_FAIL(SPH_ERR_INVALID_ARGUMENT, "NULL argument");
     const int n = s->n;
     cudaStream_t q = s->stream;
-    SPH_CUDA(cudaMemsetAsync(s->reuse, 0, sizeof(int), q));  // the state changes under the sorted copies
+    if (s->corr) SPH_CUDA(cudaMemsetAsync(s->reuse, 0, sizeof(int), q));  // the state changes under the sorted copies
     switch (field) {
         case SPH_FIELD_VERTEX_DATA:
         case SPH_FIELD_VELOCITY: {

@@ -78,15 +78,17 @@ struct sph_sim {
     // copies on a stream of their own into landing buffers (AoS), unpacked on
     // the handle's stream once landed, so the host link and the work queued
     // there overlap.  Asynchronous reads: packed on the handle's stream into
-    // a buffer of their own, copied to the host by DMA on another stream.
+    // buffers of their own, copied to the host by DMA on another stream.
     cudaStream_t upStream = nullptr;
     float* upLand[2] = {nullptr, nullptr};           // positions, velocities: float[3n]
     cudaEvent_t upReady[2] = {nullptr, nullptr};     // landed
     cudaEvent_t upFree[2] = {nullptr, nullptr};      // unpacked: the landing buffer may be refilled
     cudaStream_t downStream = nullptr;
-    float* downStage = nullptr;                      // float[3n]
-    cudaEvent_t downReady = nullptr;                 // packed
-    cudaEvent_t downFree = nullptr;                  // copied to the host: the buffer may be refilled
+    // (two buffers in turn: a second read is packed while the first is copied)
+    float* downStage[2] = {nullptr, nullptr};        // float[3n]
+    cudaEvent_t downReady[2] = {nullptr, nullptr};   // packed
+    cudaEvent_t downFree[2] = {nullptr, nullptr};    // copied to the host: the buffer may be refilled
+    int downNext = 0;
     std::vector<float> sdMass, sdEnergy;  // SD_MASS / SD_ENERGY columns (never touched by the step)
 
     // boundary maps
