@@ -342,6 +342,18 @@ static void enqueue_front(sph_sim* s, const float4* pos, const float4* vel, cons
     }
 }
 
+// Plain steps of a small handle with reused lists: whole steps in one launch.
+static bool whole_steps(const sph_sim* s) {
+    return s->vlOn && !s->sb.scenes && takes_whole_steps(s->n, (int)s->numCellsTotal);
+}
+
+static void enqueue_whole_steps(sph_sim* s, int count) {
+    launch_steps(s->n, s->pos, s->vel, grid_of(s), s->sb, rows_of(s), s->posS, s->velS, s->rho4S, s->accS,
+                 make_phys(s->P, s->O), s->map, s->O.boxCollision, s->vl, masks_of(s), s->cfg, count, s->status,
+                 s->stream);
+    s->lastStepLists = true;
+}
+
 // A plain step over the reused neighbour lists: the decision, the
 // reference's hash, sort and cell tables when some scene builds (a step that
 // builds nothing skips them; sph_read_cells builds its tables on demand),
@@ -353,6 +365,10 @@ static void enqueue_lists(sph_sim* s, const GridDev& g, const PhysDev& ph, int c
     auto mark = [&](int k) {
         if (ev) cudaEventRecord(ev[k], st);
     };
+    if (!ev && whole_steps(s)) {
+        enqueue_whole_steps(s, 1);
+        return;
+    }
     enqueue_front(s, s->pos, s->vel, g, &s->vl, ev);
     mark(ST_DENSITY);
     launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg, st);
@@ -819,6 +835,13 @@ sph_status sph_step_many(sph_handle s, int mode, int count) {
             sph_status st = sph_step(s, mode);
             if (st) return st;
         }
+        return SPH_OK;
+    }
+    if (mode == SPH_STEP_PLAIN && whole_steps(s)) {
+        enqueue_whole_steps(s, count);
+        SPH_CUDA(cudaGetLastError());
+        s->numTimeSteps += (unsigned int)count;
+        s->stepped = true;
         return SPH_OK;
     }
     if (!s->graphValid) {

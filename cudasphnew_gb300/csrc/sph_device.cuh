@@ -8,6 +8,14 @@
 
 namespace sph {
 
+// Reads memory that other blocks write in earlier phases of the same launch
+// (FRESH), or that no one writes while the kernel runs.
+template <bool FRESH, class T>
+__device__ __forceinline__ T load(const T* p) {
+    if (FRESH) return *p;
+    return __ldg(p);
+}
+
 // compute_particle_hash (particle_simulation.cu:100-115): (int) truncation,
 // C remainder, x-fastest hash.  Rounded operations are spelled out so no FMA
 // contraction can change the cell a particle falls in.
@@ -166,10 +174,11 @@ __device__ __forceinline__ bool neighbour_r2(float r2, float h2) {
 // The candidates [s, e) from cell cl of a row (its upper half on, when
 // `upperL`) to cell cr (its upper half included when `upperR`): one table
 // load an end.
+template <bool FRESH = false>
 __device__ __forceinline__ void half_cells(RowTables T, int row, int cl, int cr, bool upperL, bool upperR, int& s,
                                            int& e) {
-    s = __ldg((upperL ? T.halfOffset : T.cellOffset) + row + cl);
-    e = __ldg(upperR ? T.cellOffset + row + cr + 1 : T.halfOffset + row + cr);
+    s = load<FRESH>((upperL ? T.halfOffset : T.cellOffset) + row + cl);
+    e = load<FRESH>(upperR ? T.cellOffset + row + cr + 1 : T.halfOffset + row + cr);
     if (e < s) e = s;
 }
 
@@ -212,6 +221,7 @@ __device__ __forceinline__ void row_range(float4 xi, const Stencil& st, float h,
 // 27-cell stencil: R may exceed a cell).  The same margins as row_range, so
 // every particle within R is a candidate.  Used to build the reused
 // neighbour lists.
+template <bool FRESH>
 __device__ __forceinline__ bool row_window(float4 xi, int y, int z, float R2, float g2, float eps, const GridDev& g,
                                            RowTables T, int& s, int& e) {
     s = e = 0;
@@ -223,7 +233,7 @@ __device__ __forceinline__ bool row_window(float4 xi, int y, int z, float R2, fl
     const int cl = max(0, (int)floorf((xl - g.origin[0]) * g.inv));
     const int cr = min(g.dim[0] - 1, (int)floorf((xr - g.origin[0]) * g.inv));
     if (cl > cr) return false;
-    half_cells(T, g.cellBase + g.dim[0] * (g.dim[1] * z + y), cl, cr,
+    half_cells<FRESH>(T, g.cellBase + g.dim[0] * (g.dim[1] * z + y), cl, cr,
                xl >= g.origin[0] + ((float)cl + 0.5f) * g.spacing, xr >= g.origin[0] + ((float)cr + 0.5f) * g.spacing, s,
                e);
     return e > s;

@@ -249,6 +249,14 @@ constexpr int FRONT_MAX_BLOCKS = 4088;
 constexpr int FRONT_WORDS = FRONT_MAX_BLOCKS + 8;
 void launch_front(int n, const float4* pos, const float4* vel, GridDev g, SortBuffers sb, float4* posS, float4* velS,
                   unsigned int* status, cudaStream_t s, const NeighbourLists* lists = nullptr, int phases = FRONT_ALL);
+// The poll limit of device-side waits (a test may shorten it).
+int scan_wait_limit();
+// `steps` whole plain steps over the reused lists (single scene, absolute
+// positions): in one launch after another of several steps each.
+bool takes_whole_steps(int n, int numCells);
+void launch_steps(int n, float4* pos, float4* vel, GridDev g, SortBuffers sb, RowTables T, float4* posS, float4* velS,
+                  float4* rho4S, float4* accS, PhysDev ph, MapDev map, int collide, const NeighbourLists& L, RowMasks M,
+                  const StepConfig& cfg, int steps, unsigned int* status, cudaStream_t s);
 // The fine level's cell offsets (two-scale pass).
 void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s);
 // The cell tables of the sorted copies' positions (sortedHash, sortedIds,

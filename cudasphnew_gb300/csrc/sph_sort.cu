@@ -12,13 +12,10 @@
 // cell with one atomic, a scan turns counts into cell offsets, and a rank pass
 // orders each cell's members by particle id.  The result is the permutation of a stable sort by hash -- the order
 // thrust::sort_by_key produces in the reference (particle_simulation.cu:2340).
-#include <cuda/atomic>
-
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 
-#include "sph_device.cuh"
+#include "sph_front.cuh"
 
 namespace sph {
 
@@ -275,7 +272,7 @@ k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, unsigned lo
 // variable SPH_SCAN_WAIT_LIMIT (read at each launch; a captured step graph
 // keeps the value it was captured with).  Tests set it to exercise the
 // give-up path; -1 abandons every wait at once.
-static int scan_wait_limit() {
+int scan_wait_limit() {
     const char* e = getenv("SPH_SCAN_WAIT_LIMIT");
     if (!e || !*e) return SPIN_LIMIT;
     return (int)strtol(e, nullptr, 10);
@@ -338,319 +335,14 @@ void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaSt
 // ---------------------------------------------------------------------------
 constexpr int FRONT_THREADS = 512;
 constexpr int FRONT_WIDE = 1 << 19;
-constexpr int FRONT_WARPS = FRONT_THREADS / 32;
-// words of SortBuffers::front: barrier arrivals, blocks gone, a wait gave up, then the blocks' sums
-enum : int { FRONT_ARRIVED = 0, FRONT_GONE = 1, FRONT_FAILED = 2, FRONT_SUMS = 8 };
-
-struct FrontArgs {
-    int n;
-    const float4* pos;
-    const float4* vel;
-    GridDev g;
-    SortBuffers sb;
-    float4* posS;
-    float4* velS;
-    unsigned int* status;
-    NeighbourLists L;
-    int lists;
-    int phases;
-    int waitLimit;
-};
-
-__device__ __forceinline__ unsigned int ordered_bits(float x) {
-    unsigned int u = __float_as_uint(x);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// Waits until every block of the grid has arrived `round` times.
-__device__ __forceinline__ bool grid_barrier(unsigned int* front, unsigned int round, int waitLimit, unsigned int* status) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> arrived(front[FRONT_ARRIVED]);
-        arrived.fetch_add(1u, cuda::memory_order_acq_rel);
-        const unsigned int all = round * gridDim.x;
-        int spins = 0;
-        ok = 1;
-        while (arrived.load(cuda::memory_order_acquire) < all || waitLimit < 0) {
-            if (++spins > waitLimit) {
-                ok = 0;
-                atomicOr(status, STATUS_DEVICE_WAIT);
-                atomicExch(front + FRONT_FAILED, 1u);
-                break;
-            }
-            __nanosleep(20);
-        }
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-__device__ __forceinline__ int front_block_sum(int v, int* warps) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int t = 0;
-#pragma unroll
-    for (int w = 0; w < FRONT_WARPS; w++) t += warps[w];
-    return t;
-}
-
-// What kind of step a scene takes: VL_BUILDS on request or when a particle
-// has moved farther than the skin allows since the last build (or the
-// displacement is not finite), VL_SEARCHES in place of a build that the last
-// step's own displacement would have outrun.
-__device__ __forceinline__ unsigned int list_kind(const NeighbourLists& L, const SceneDev* __restrict__ scenes, int k) {
-    const int S = L.numScenes;
-    const unsigned int* f = L.flags;
-    float lim2 = L.dispLimit2;
-    if (scenes) {
-        const float lim = 0.45f * L.skinFrac * scenes[k].ph.h;
-        lim2 = lim * lim;
-    }
-    if (f[VL_BUILD * S + k]) return VL_BUILDS;
-    const unsigned int last = f[VL_LAST * S + k];
-    if (!(__uint_as_float(f[VL_DISP * S + k]) <= lim2)) return last == VL_REUSES ? VL_BUILDS : VL_SEARCHES;
-    return last == VL_SEARCHES ? VL_BUILDS : VL_REUSES;
-}
-
-template <bool BATCH>
-__device__ __forceinline__ void front_gather(const FrontArgs& A) {
-    for (int k = blockIdx.x * FRONT_THREADS + threadIdx.x; k < A.n; k += gridDim.x * FRONT_THREADS) {
-        const int w = A.sb.workIds[k];
-        const float4 p = __ldg(A.pos + w), v = __ldg(A.vel + w);
-        A.posS[k] = p;
-        A.velS[k] = v;
-        const GridDev& g = BATCH ? A.sb.scenes[A.L.slotScene[k]].g : A.g;
-        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) {
-            atomicOr(A.status, STATUS_NON_FINITE);
-        } else {
-            bool outside = false;
-            particle_hash(p, g, &outside);
-            if (outside) atomicOr(A.status, STATUS_OUT_OF_DOMAIN);
-        }
-    }
-}
-
-// BATCH: the particle's scene (pos.w) supplies its grid, whose cells start at
-// that scene's cellBase in the concatenated cell space.  REL: the position is
-// cell-relative and the hash comes from its packed cell coordinates.
-template <bool BATCH, bool REL>
-__device__ __forceinline__ void front_hash(const FrontArgs& A) {
-    for (int i = blockIdx.x * FRONT_THREADS + threadIdx.x; i < A.n; i += gridDim.x * FRONT_THREADS) {
-        float4 p = A.pos[i];
-        const GridDev& g = BATCH ? A.sb.scenes[__float_as_int(p.w)].g : A.g;
-        bool outside = false;
-        const bool finite = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
-        if (!finite) {
-            atomicOr(A.status, STATUS_NON_FINITE);
-            p = make_float4(g.origin[0], g.origin[1], g.origin[2], 0.f);
-        }
-        int h;
-        if (REL) {
-            const int3 c = finite ? rel_cell(p) : make_int3(0, 0, 0);
-            h = g.cellBase + g.dim[0] * (g.dim[1] * c.z + c.y) + c.x;
-        } else {
-            h = particle_hash(p, g, &outside);
-        }
-        if (outside) atomicOr(A.status, STATUS_OUT_OF_DOMAIN);
-        A.sb.keySlot[i] = make_int2(h, atomicAdd(A.sb.cnt + h, 1));
-    }
-}
-
-template <bool BATCH, bool REL>
-__device__ __forceinline__ void front_rank(const FrontArgs& A) {
-    // (plain loads: what earlier phases of this launch wrote)
-    for (int k = blockIdx.x * FRONT_THREADS + threadIdx.x; k < A.n; k += gridDim.x * FRONT_THREADS) {
-        const int c = A.sb.sortedHash[k];
-        const int s = A.sb.cellOffset[c], e = A.sb.cellOffset[c + 1];
-        const int my = A.sb.tmpIds[k];
-        if (A.lists && A.L.flags[VL_BUILD_NOW * A.L.numScenes + (BATCH ? A.L.slotScene[k] : 0)] == VL_REUSES) {
-            int rId = 0;
-            for (int t = s; t < e; t++) rId += A.sb.tmpIds[t] < my;
-            A.sb.sortedIds[s + rId] = my;
-            const int w = A.sb.workIds[k];
-            A.posS[k] = __ldg(A.pos + w);
-            A.velS[k] = __ldg(A.vel + w);
-            continue;
-        }
-        const float4 p = __ldg(A.pos + my);
-        const GridDev& g = BATCH ? A.sb.scenes[__float_as_int(p.w)].g : A.g;
-        const unsigned int key = ordered_bits(p.x);
-        // the cell's mid-plane, in the frame its members' x is stored in
-        const float mid = REL ? 0.5f * g.spacing
-                              : g.origin[0] + ((float)((c - g.cellBase) % g.dim[0]) + 0.5f) * g.spacing;
-        int rId = 0, rX = 0, below = 0;
-        for (int t = s; t < e; t++) {
-            const int o = A.sb.tmpIds[t];
-            const float xo = __ldg(&A.pos[o].x);
-            const unsigned int ko = ordered_bits(xo);
-            rId += o < my;
-            rX += (ko < key) || (ko == key && o < my);
-            below += xo < mid;
-        }
-        A.sb.sortedIds[s + rId] = my;
-        A.sb.workIds[s + rX] = my;
-        A.posS[s + rX] = p;
-        A.velS[s + rX] = __ldg(A.vel + my);
-        if (rX == 0) A.sb.halfOffset[c] = s + below;
-    }
-}
 
 template <bool BATCH, bool REL>
 __global__ void __launch_bounds__(FRONT_THREADS, 3) k_front(FrontArgs A) {
-    __shared__ int warps[FRONT_WARPS];
-    __shared__ int carry;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    unsigned int* front = A.sb.front;
     if (A.sb.skip && *A.sb.skip) return;
-    bool ok = !(*(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT);
-    unsigned int* f = A.L.flags;
-    const int S = A.L.numScenes;
-    if (ok && A.lists) {
-        // The decision, or (a launch of later phases alone) what it was.  What
-        // it is taken from changes with the rank phase, when every block has
-        // decided (where nothing sorts, to what gives the same decision again).
-        bool sorts = false;
-        if (A.phases & FRONT_HASH) {
-            for (int k = t; k < S; k += FRONT_THREADS) {
-                const unsigned int kind = list_kind(A.L, A.sb.scenes, k);
-                sorts |= kind != VL_REUSES;
-                if (blockIdx.x == 0) f[VL_BUILD_NOW * S + k] = kind;
-            }
-            sorts = __syncthreads_or(sorts);
-            if (blockIdx.x == 0 && t == 0) {
-                f[VL_FLAGS * S + VL_SORT] = sorts ? 1u : 0u;
-                f[VL_FLAGS * S + VL_STALE] = sorts ? 0u : 1u;
-            }
-        } else {
-            sorts = f[VL_FLAGS * S + VL_SORT] != 0u;
-        }
-        if (!sorts) {
-            if (!(A.phases & FRONT_RANK)) return;
-            if (blockIdx.x == 0)
-                for (int k = t; k < S; k += FRONT_THREADS) f[VL_LAST * S + k] = VL_REUSES;
-            front_gather<BATCH>(A);
-            return;
-        }
-    }
     unsigned int round = 0;
-    auto barrier = [&]() { ok = grid_barrier(front, ++round, A.waitLimit, A.status); };
-    if (ok && (A.phases & FRONT_HASH)) {
-        front_hash<BATCH, REL>(A);
-        if (A.phases & FRONT_SCAN) barrier();
-    }
-    // this block's stretch of cells, four at a time (the buffers are padded)
-    const long long total = ((long long)A.g.numCells + 4) & ~3ll;  // numCells + 1 counts
-    const long long per = ((total / 4 + gridDim.x - 1) / gridDim.x) * 4;
-    const long long c0 = per * blockIdx.x, c1 = min(c0 + per, total);
-    if (ok && (A.phases & FRONT_SUM)) {
-        int sum = 0;
-        for (long long c = c0 + 4 * t; c < c1; c += 4 * FRONT_THREADS) {
-            const int4 v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
-            sum += v.x + v.y + v.z + v.w;
-        }
-        sum = front_block_sum(sum, warps);
-        if (t == 0) front[FRONT_SUMS + blockIdx.x] = (unsigned int)sum;
-        barrier();
-    }
-    if (ok && (A.phases & FRONT_SCAN)) {
-        int before = 0;
-        for (int b = t; b < (int)blockIdx.x; b += FRONT_THREADS) before += (int)front[FRONT_SUMS + b];
-        before = front_block_sum(before, warps);
-        for (long long base = c0; base < c1; base += 4 * FRONT_THREADS) {
-            const long long c = base + 4 * t;
-            int4 v = make_int4(0, 0, 0, 0);
-            if (c < c1) {
-                v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
-                *reinterpret_cast<int4*>(A.sb.cnt + c) = make_int4(0, 0, 0, 0);
-            }
-            const int local = v.x + v.y + v.z + v.w;
-            int incl = local;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += u;
-            }
-            __syncthreads();  // (the last use of `warps` and `carry`)
-            if (lane == 31) warps[warp] = incl;
-            __syncthreads();
-            int run = before + incl - local;
-            for (int w = 0; w < warp; w++) run += warps[w];
-            if (t == FRONT_THREADS - 1) carry = run + local;
-            if (c < c1) {
-                int4 o;
-                o.x = run;
-                o.y = o.x + v.x;
-                o.z = o.y + v.y;
-                o.w = o.z + v.z;
-                *reinterpret_cast<int4*>(A.sb.cellOffset + c) = o;
-                if (A.sb.halfOffset) *reinterpret_cast<int4*>(A.sb.halfOffset + c) = o;
-            }
-            __syncthreads();
-            before = carry;
-        }
-        if (A.phases & FRONT_SCATTER) barrier();
-    }
-    if (ok && (A.phases & FRONT_SCATTER)) {
-        for (int i = blockIdx.x * FRONT_THREADS + t; i < A.n; i += gridDim.x * FRONT_THREADS) {
-            const int2 ks = A.sb.keySlot[i];
-            const int dst = A.sb.cellOffset[ks.x] + ks.y;
-            A.sb.tmpIds[dst] = i;
-            A.sb.sortedHash[dst] = ks.x;
-        }
-        if (A.phases & FRONT_RANK) barrier();
-    }
-    if (ok && (A.phases & FRONT_RANK)) {
-        if (A.lists && blockIdx.x == 0) {
-            for (int k = t; k < S; k += FRONT_THREADS) {
-                const unsigned int kind = f[VL_BUILD_NOW * S + k];
-                f[VL_LAST * S + k] = kind;
-                f[VL_BUILD * S + k] = 0u;
-                if (kind != VL_REUSES) {
-                    f[VL_DISP * S + k] = 0u;
-                    if (kind == VL_BUILDS) f[VL_COUNT * S + k] += 1u;
-                }
-            }
-        }
-        front_rank<BATCH, REL>(A);
-    }
-    // the last block to leave readies the words for the next launch
-    __syncthreads();
-    if (t == 0) {
-        __threadfence();
-        carry = atomicAdd(front + FRONT_GONE, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (!carry) return;
-    __threadfence();
-    if (*(volatile unsigned int*)(front + FRONT_FAILED)) {
-        for (long long c = t; c < total; c += FRONT_THREADS) A.sb.cnt[c] = 0;
-        if (A.lists)
-            for (int k = t; k < S; k += FRONT_THREADS) f[VL_BUILD * S + k] = 1u;
-    }
-    __syncthreads();
-    if (t < FRONT_SUMS) front[t] = 0u;
-}
-
-// `perSm` blocks of k_front an SM, as far as the current device holds them at once.
-template <bool BATCH, bool REL>
-static int front_resident(int perSm) {
-    static std::atomic<int> known[64];  // blocks an SM times 4096, plus SMs
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int k = dev < 64 ? known[dev].load() : 0;
-    if (k == 0) {
-        int fit = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_front<BATCH, REL>, FRONT_THREADS, 0) != cudaSuccess ||
-            fit < 1)
-            fit = 1;
-        k = fit * 4096 + std::min(device_sms(), 4095);
-        if (dev < 64) known[dev].store(k);
-    }
-    return std::min(std::min(perSm, k / 4096) * (k % 4096), FRONT_MAX_BLOCKS);
+    bool ok = !(*(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT);
+    front_phases<BATCH, REL, FRONT_THREADS, false>(A, round, ok);
+    if (round || !ok) front_leave<FRONT_THREADS>(A);
 }
 
 template <bool BATCH, bool REL>
@@ -658,7 +350,7 @@ static void front_launch(FrontArgs A, cudaStream_t s) {
     // one particle a thread and sixteen cells, as far as the blocks may be
     const long long want = std::max(((long long)A.n + FRONT_THREADS - 1) / FRONT_THREADS,
                                     ((long long)A.g.numCells + 16 * FRONT_THREADS) / (16 * FRONT_THREADS));
-    const int most = front_resident<BATCH, REL>(A.n > FRONT_WIDE ? 2 : 1);
+    const int most = resident_blocks<k_front<BATCH, REL>>(FRONT_THREADS, A.n > FRONT_WIDE ? 2 : 1);
     const int grid = (int)std::max(1ll, std::min(want, (long long)most));
     void* args[] = {&A};
     cudaLaunchCooperativeKernel((const void*)k_front<BATCH, REL>, dim3(grid), dim3(FRONT_THREADS), args, 0, s);

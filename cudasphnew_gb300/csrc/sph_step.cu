@@ -18,9 +18,10 @@
 //                records each row's window start and a 32-bit neighbour mask;
 //                the force stage runs the interactions of the set bits only
 //                (rows longer than 32 candidates fall back to testing).
+#include <algorithm>
 #include <climits>
 
-#include "sph_device.cuh"
+#include "sph_front.cuh"
 #include "sph_mlp_tile.cuh"
 
 namespace sph {
@@ -41,13 +42,13 @@ __device__ __forceinline__ bool within_r2(float r2, float R2) {  // r2 >= 0 or N
 // in flight together and their bits put together from constants (230 against
 // 254 us for the list build of a million particles, 21 against 27 at 16,384).
 // REL: positions are cell-relative and moved into particle i's frame.
-template <bool REL, bool SKIN>
-__device__ __forceinline__ void row_tests(const float4* __restrict__ posS, int base, int c, float4 xi, float h2,
+template <bool REL, bool SKIN, bool FRESH>
+__device__ __forceinline__ void row_tests(const float4* posS, int base, int c, float4 xi, float h2,
                                           float R2, int cx, float dyo, float dzo, float spacing, float& rs,
                                           unsigned int& mR, unsigned int& mh) {
     mR = mh = 0u;
     auto at = [&](const float4* p) {
-        const float4 x = __ldg(p);
+        const float4 x = load<FRESH>(p);
         return REL ? rel_in_frame(x, cx, dyo, dzo, spacing) : x;
     };
     const float4* p = posS + base;
@@ -117,7 +118,7 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
         float rs = 0.f;
         unsigned int m = 0u, mR;
         for (int base = s; base < e; base += 32)
-            row_tests<REL, false>(posS, base, min(32, e - base), xi, h2, 0.f, ci.x, dyo, dzo, g.spacing, rs, mR, m);
+            row_tests<REL, false, false>(posS, base, min(32, e - base), xi, h2, 0.f, ci.x, dyo, dzo, g.spacing, rs, mR, m);
         if (KAHAN) {
             if (rs > 0.f) kahan_add(sum, comp, rs);
         } else {
@@ -145,10 +146,10 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
 //
 // Build form (steps that build the lists): every row that the skin sphere of
 // radius R reaches, in the reference's order, its window at R walked in the
-// working order.  The reference's own 3 x 3 rows give the density terms, summed as in k_density (candidates
-// beyond h add exactly nothing, so the row sums are the same), and this
-// step's neighbours by row for the force stage; every row gives its
-// candidates within R to the particle's list.  A step that searches without
+// working order.  The reference's own 3 x 3 rows give the density terms,
+// summed as in k_density (candidates beyond h add exactly nothing, so the row
+// sums are the same), and this step's neighbours by row for the force stage;
+// every row gives its candidates within R to the particle's list.  A step that searches without
 // building (VL_SEARCHES) takes windows at h and records those.
 //
 // A row is tested 32 candidates at a time into two bit masks (within R,
@@ -159,7 +160,9 @@ k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysD
 // misses L1 (184 of 302 sectors a warp in the density stage), so they leave no
 // lines there (1,048,576 particles: density 61.6 -> 58.8 us; a batch of 16
 // scenes: density 41.0 -> 39.0, force 74.0 -> 67.7).
+template <bool FRESH>
 __device__ __forceinline__ int4 load_group(const int4* p) {
+    if (FRESH) return *p;
     int4 c;
     asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
         : "=r"(c.x), "=r"(c.y), "=r"(c.z), "=r"(c.w)
@@ -168,12 +171,11 @@ __device__ __forceinline__ int4 load_group(const int4* p) {
 }
 
 // BATCH: the slot's scene supplies grid, constants, maps and R.
-template <bool KAHAN, bool BATCH>
+template <bool KAHAN, bool BATCH, bool FRESH>
 __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int scene, float4* posS, float4* velS,
                                                   const RowTables& T,
                                                   const GridDev& g_, const PhysDev& ph_, const MapDev& map_,
-                                                  float4* __restrict__ rho4S, const NeighbourLists& L,
-                                                  const RowMasks& M) {
+                                                  float4* rho4S, const NeighbourLists& L, const RowMasks& M) {
     const float4 xi = posS[i];
     const SceneDev* S = BATCH ? T.scenes + scene : nullptr;
     const GridDev& g = BATCH ? S->g : g_;
@@ -204,7 +206,7 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
             for (int y = ya; y <= yb; y++) {
                 const float gy = cell_gap(xi.y, y, g.origin[1], g.spacing, eps);
                 int s, e;
-                if (row_window(xi, y, z, reach2, gy * gy + gz * gz, eps, g, T, s, e)) row(y, z, s, e);
+                if (row_window<FRESH>(xi, y, z, reach2, gy * gy + gz * gz, eps, g, T, s, e)) row(y, z, s, e);
             }
         }
     };
@@ -216,7 +218,7 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
         unsigned int m = 0u;  // neighbours within h, bit t - first
         for (int base = s0; base < e0; base += 32) {
             unsigned int mR, mh;
-            row_tests<false, true>(posS, base, min(32, e0 - base), xi, h2, R2, 0, 0.f, 0.f, 0.f, rs, mR, mh);
+            row_tests<false, true, FRESH>(posS, base, min(32, e0 - base), xi, h2, R2, 0, 0.f, 0.f, 0.f, rs, mR, mh);
             if (mh) {
                 if (first < 0) {
                     const int k = __ffs(mh) - 1;
@@ -288,16 +290,14 @@ constexpr int DENSITY_LIST_BLOCKS = 4;
 // summed in plain FP32 (as a row's few terms are) and the group sums are
 // added with compensation.  The next group's slots are loaded before the
 // current group's positions are used.
-template <bool KAHAN, bool BATCH>
-__global__ void __launch_bounds__(256, DENSITY_LIST_BLOCKS)
-k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph_, MapDev map_,
-                float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+template <bool KAHAN, bool BATCH, bool FRESH>
+__device__ __forceinline__ void density_list_one(int i, int n, float4* posS, float4* velS, const RowTables& T,
+                                                 const GridDev& g, const PhysDev& ph_, const MapDev& map_,
+                                                 float4* rho4S, const NeighbourLists& L, const RowMasks& M) {
     const int scene = BATCH ? L.slotScene[i] : 0;
     const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
     if (kind != VL_REUSES) {
-        density_build_one<KAHAN, BATCH>(i, n, kind == VL_BUILDS, scene, posS, velS, T, g, ph_, map_, rho4S, L, M);
+        density_build_one<KAHAN, BATCH, FRESH>(i, n, kind == VL_BUILDS, scene, posS, velS, T, g, ph_, map_, rho4S, L, M);
         return;
     }
     const float4 xi = posS[i];
@@ -312,13 +312,13 @@ k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysD
     };
     if (!(groups & VL_WINDOWS)) {
         const int4* lp = L.list + i;
-        int4 c = groups ? load_group(lp) : make_int4(0, 0, 0, 0);
+        int4 c = groups ? load_group<FRESH>(lp) : make_int4(0, 0, 0, 0);
 #pragma unroll 1
         for (unsigned int k = 0; k < groups; k++) {
-            const float4 x0 = __ldg(posS + c.x), x1 = __ldg(posS + c.y), x2 = __ldg(posS + c.z),
-                         x3 = __ldg(posS + c.w);
+            const float4 x0 = load<FRESH>(posS + c.x), x1 = load<FRESH>(posS + c.y), x2 = load<FRESH>(posS + c.z),
+                         x3 = load<FRESH>(posS + c.w);
             lp += n;
-            if (k + 1 < groups) c = load_group(lp);
+            if (k + 1 < groups) c = load_group<FRESH>(lp);
             const float w0 = fmaxf(h2 - dist2(xi, x0), 0.f), w1 = fmaxf(h2 - dist2(xi, x1), 0.f);
             const float w2 = fmaxf(h2 - dist2(xi, x2), 0.f), w3 = fmaxf(h2 - dist2(xi, x3), 0.f);
             total(fmaf(w3 * w3, w3, fmaf(w2 * w2, w2, fmaf(w1 * w1, w1, w0 * w0 * w0))));
@@ -329,7 +329,7 @@ k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysD
             const int2 se = list_window(L, n, i, (int)w);
             float rs = 0.f;
             for (int t = se.x; t < se.y; t++) {
-                const float d = fmaxf(h2 - dist2(xi, __ldg(posS + t)), 0.f);
+                const float d = fmaxf(h2 - dist2(xi, load<FRESH>(posS + t)), 0.f);
                 rs = fmaf(d * d, d, rs);
             }
             total(rs);
@@ -348,6 +348,14 @@ k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysD
     // velocity rides in their unused fourth lanes: two loads per pair, not three
     posS[i].w = p * inv * inv;
     velS[i].w = inv;
+}
+
+template <bool KAHAN, bool BATCH>
+__global__ void __launch_bounds__(256, DENSITY_LIST_BLOCKS)
+k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
+                float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) density_list_one<KAHAN, BATCH, false>(i, n, posS, velS, T, g, ph, map, rho4S, L, M);
 }
 
 // The far record: r^2 of any particle to it is ~3e36, beyond every support
@@ -382,6 +390,9 @@ struct Pair {
     }
 };
 
+// (sums of two products are spelled as fmaf here and in force_finish: which
+// of the two the compiler fuses may differ between kernels, and every form of
+// the stage gives the same bits)
 template <bool TENSION>
 struct RowSums {
     float fp[3], fv[3], cg[3], cl;
@@ -410,7 +421,7 @@ struct RowSums {
             cg[0] = fmaf(sc, p.dx, cg[0]);
             cg[1] = fmaf(sc, p.dy, cg[1]);
             cg[2] = fmaf(sc, p.dz, cg[2]);
-            cl = fmaf(rj.w * d2, 3.f * ph.h2 - 7.f * p.r2, cl);
+            cl = fmaf(rj.w * d2, fmaf(-7.f, p.r2, 3.f * ph.h2), cl);
         }
         if (COUNT) hits++;
     }
@@ -567,7 +578,7 @@ __device__ __forceinline__ void force_finish(const ForceTotals<KAHAN, TENSION>& 
     for (int a = 0; a < 3; a++) {
         const float P = KAHAN ? __fsub_rn(A.fp[a], A.cp[a]) : A.fp[a];
         const float V = KAHAN ? __fsub_rn(A.fv[a], A.cv[a]) : A.fv[a];
-        force[a] = ph.viscCoef * V + pc * P;
+        force[a] = fmaf(pc, P, ph.viscCoef * V);
     }
     bool tension = TENSION;
     if (map.present) {
@@ -607,7 +618,7 @@ __device__ __forceinline__ void force_finish(const ForceTotals<KAHAN, TENSION>& 
     }
     if (TENSION && tension) {
         const float cgx = ph.cgCoef * A.cg[0], cgy = ph.cgCoef * A.cg[1], cgz = ph.cgCoef * A.cg[2];
-        const float norm = sqrtf(cgx * cgx + cgy * cgy + cgz * cgz);
+        const float norm = sqrtf(fmaf(cgz, cgz, fmaf(cgy, cgy, cgx * cgx)));
         if (norm > ph.normThresh) {
             const float fc = ph.tension * (ph.clCoef * A.cl) / norm;
             force[0] -= fc * cgx;
@@ -826,30 +837,30 @@ __global__ void __launch_bounds__(256, FEAT ? 3 : (BATCH || TENSION || REL || FO
 // The neighbours of a list step's particle: `pair` for each candidate (with
 // `tested` when it is known to lie within h), `row` with the sums of each
 // row's, window's or (group true) list group's pairs.
-template <bool TENSION, class PAIR, class ROW>
+template <bool TENSION, bool FRESH, class PAIR, class ROW>
 __device__ __forceinline__ void list_rows(int i, int n, int scene, const NeighbourLists& L, const RowMasks& M,
-                                          const float4* __restrict__ posS, const float4* __restrict__ velS,
+                                          const float4* posS, const float4* velS,
                                           PAIR&& pair, ROW&& row) {
     if (L.flags[VL_BUILD_NOW * L.numScenes + scene]) {
-        int svN = __ldg(M.start + i);
-        unsigned int mN = __ldg(M.mask + i);
+        int svN = load<FRESH>(M.start + i);
+        unsigned int mN = load<FRESH>(M.mask + i);
 #pragma unroll 1
         for (int r = 0; r < 9; r++) {
             const int sv = svN;
             unsigned int m = mN;
             if (r + 1 < 9) {
-                svN = __ldg(M.start + (size_t)(r + 1) * n + i);
-                mN = __ldg(M.mask + (size_t)(r + 1) * n + i);
+                svN = load<FRESH>(M.start + (size_t)(r + 1) * n + i);
+                mN = load<FRESH>(M.mask + (size_t)(r + 1) * n + i);
             }
             RowSums<TENSION> R;
             R.clear();
             if (sv < 0) {
-                for (int t = sv & 0x7fffffff; t < (int)m; t++) pair(R, __ldg(posS + t), __ldg(velS + t), false);
+                for (int t = sv & 0x7fffffff; t < (int)m; t++) pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), false);
             } else {
                 while (m) {
                     const int t = sv + __ffs(m) - 1;
                     m &= m - 1u;
-                    pair(R, __ldg(posS + t), __ldg(velS + t), true);
+                    pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
                 }
             }
             row(R, false);
@@ -863,19 +874,19 @@ __device__ __forceinline__ void list_rows(int i, int n, int scene, const Neighbo
             const int2 se = list_window(L, n, i, (int)w);
             RowSums<TENSION> R;
             R.clear();
-            for (int t = se.x; t < se.y; t++) pair(R, __ldg(posS + t), __ldg(velS + t), false);
+            for (int t = se.x; t < se.y; t++) pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), false);
             row(R, false);
         }
         return;
     }
     const int4* lp = L.list + i;
-    int4 c = groups ? load_group(lp) : make_int4(0, 0, 0, 0);
+    int4 c = groups ? load_group<FRESH>(lp) : make_int4(0, 0, 0, 0);
 #pragma unroll 1
     for (unsigned int k = 0; k < groups; k++) {
-        const float4 x0 = __ldg(posS + c.x), x1 = __ldg(posS + c.y), x2 = __ldg(posS + c.z), x3 = __ldg(posS + c.w);
-        const float4 v0 = __ldg(velS + c.x), v1 = __ldg(velS + c.y), v2 = __ldg(velS + c.z), v3 = __ldg(velS + c.w);
+        const float4 x0 = load<FRESH>(posS + c.x), x1 = load<FRESH>(posS + c.y), x2 = load<FRESH>(posS + c.z), x3 = load<FRESH>(posS + c.w);
+        const float4 v0 = load<FRESH>(velS + c.x), v1 = load<FRESH>(velS + c.y), v2 = load<FRESH>(velS + c.z), v3 = load<FRESH>(velS + c.w);
         lp += n;
-        if (k + 1 < groups) c = load_group(lp);
+        if (k + 1 < groups) c = load_group<FRESH>(lp);
         RowSums<TENSION> R;
         R.clear();
         pair(R, x0, v0, false);
@@ -886,9 +897,10 @@ __device__ __forceinline__ void list_rows(int i, int n, int scene, const Neighbo
     }
 }
 
-#ifndef FORCE_REGS
-#define FORCE_REGS 72
-#endif
+// What bounds the reusing form at 1,048,576 particles: the L1 data pipe (78 %
+// busy with two gathers of 16 bytes a pair), then issue (53 %).  Registers a
+// thread, and what the stage takes: 64 (spills) 131 us, 72 109 us, 80 115 us.
+constexpr int FORCE_REGS = 72;
 // Displacement since the build into the scene's flag: one atomic per warp (or
 // per scene a warp holds) that raises the recorded maximum.  Squared
 // distances are non-negative, so their bits order as the values do; the
@@ -904,13 +916,13 @@ __device__ __forceinline__ void record_displacement(const NeighbourLists& L, int
         atomicMax(f, w);
 }
 
-template <bool KAHAN, bool TENSION, bool BATCH>
-__global__ void __maxnreg__(FORCE_REGS)
-k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__ velS,
-              const float4* __restrict__ rho4S, const int* __restrict__ workIds, PhysDev ph_, MapDev map_,
-              int collideFlag, NeighbourLists L, RowMasks M, float4* __restrict__ pos, float4* __restrict__ vel,
-              float4* __restrict__ accS, const SceneDev* __restrict__ scenes) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// (every thread of the warp calls it: i may lie beyond the particles)
+template <bool KAHAN, bool TENSION, bool BATCH, bool FRESH>
+__device__ __forceinline__ void force_list_one(int i, int n, const float4* posS, const float4* velS,
+                                               const float4* rho4S, const int* workIds, const PhysDev& ph_,
+                                               const MapDev& map_, int collideFlag, const NeighbourLists& L,
+                                               const RowMasks& M, float4* pos, float4* vel, float4* accS,
+                                               const SceneDev* scenes) {
     float d2 = 0.f;
     int scene = 0;
     if (i < n) {
@@ -924,12 +936,21 @@ k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__
         ForceTotals<KAHAN, TENSION> A;
         // (a neighbour's p/rho^2 and 1/rho ride in the fourth lanes of its
         // sorted position and velocity, written by the density stage)
-        list_rows<TENSION>(
+        list_rows<TENSION, FRESH>(
             i, n, scene, L, M, posS, velS,
             [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
-                const Pair p(ph, xi, vi, xj, vj);
-                if (tested || neighbour_r2(p.r2, h2))
+                Pair p(ph, xi, vi, xj, vj);
+                const bool in = tested || neighbour_r2(p.r2, h2);
+                if (FRESH) {  // (a pair out of reach adds zeros)
+                    if (!in) {
+                        p.r2 = h2;
+                        p.hr = p.rinv = p.dx = p.dy = p.dz = p.ux = p.uy = p.uz = xj.w = vj.w = 0.f;
+                    }
+                    R.template add<false>(ph, p, ri.z, make_float4(0.f, 0.f, xj.w, vj.w));
+                    R.hits += in;
+                } else if (in) {
                     R.add(ph, p, ri.z, make_float4(0.f, 0.f, xj.w, vj.w));
+                }
             },
             [&](const RowSums<TENSION>& R, bool group) {
                 if (group) A.add_all(R);
@@ -944,12 +965,91 @@ k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__
         pos[id] = make_float4(x.x, x.y, x.z, BATCH ? __int_as_float(scene) : 0.f);
         vel[id] = make_float4(v.x, v.y, v.z, 0.f);
         accS[i] = make_float4(acc[0], acc[1], acc[2], 0.f);
-        const float4 b = __ldg(L.posB + i);
+        const float4 b = load<FRESH>(L.posB + i);
         const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
         d2 = dx * dx + dy * dy + dz * dz;
         if (!(d2 == d2)) d2 = __uint_as_float(0x7f800000u);  // NaN: as far as it gets
     }
     record_displacement<BATCH>(L, scene, d2);
+}
+
+template <bool KAHAN, bool TENSION, bool BATCH>
+__global__ void __maxnreg__(FORCE_REGS)
+k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__ velS,
+              const float4* __restrict__ rho4S, const int* __restrict__ workIds, PhysDev ph, MapDev map,
+              int collideFlag, NeighbourLists L, RowMasks M, float4* __restrict__ pos, float4* __restrict__ vel,
+              float4* __restrict__ accS, const SceneDev* __restrict__ scenes) {
+    force_list_one<KAHAN, TENSION, BATCH, false>(blockIdx.x * blockDim.x + threadIdx.x, n, posS, velS, rho4S, workIds,
+                                                 ph, map, collideFlag, L, M, pos, vel, accS, scenes);
+}
+
+// ---------------------------------------------------------------------------
+// Whole steps over the reused lists in one cooperative launch, for handles of
+// few particles.  What bounds a step of 16,384 particles is no unit of the
+// chip but the latency of what follows one another: three launches, and in
+// each one wave of warps that walk their lists.  Here the phases of the front,
+// the density stage and the force stage are set apart by grid barriers (1.0 to
+// 1.5 us each, against 2 to 3 for a launch that waits for the one before), and
+// a call of many steps takes up to STEPS_A_LAUNCH of them a launch.  A step
+// alone on the chip, and with three handles in turn, in us, before and now:
+//   4,096   24.8 -> 21.0    9.4 -> 7.4
+//   16,384  25.5 -> 20.6   10.2 -> 8.4
+//   24,576  26.6 -> 23.2   11.0 -> 9.7
+//   32,768  27.5 -> 23.0   11.8 -> 14.5
+// (three 32,768-particle grids no longer fit the chip side by side and wait
+// for one another: the line is drawn below that).  More list groups in flight
+// a thread (2 to 8, at 140 to 200 registers) gave nothing.
+// A grid of more cells than STEPS_CELLS is left to k_front, whose blocks are
+// four times as large: the scan of a building step walks every cell.
+// The stages are the kernels' own functions and give the same bits; FRESH:
+// what one phase writes another reads in the same launch, so no read goes
+// through the read-only path, and the few warps that run evaluate every pair
+// without a branch (4 % of a step: a group's four pairs overlap).
+// ---------------------------------------------------------------------------
+constexpr int STEPS_PARTICLES = 24576;
+constexpr int STEPS_CELLS = 1 << 18;
+constexpr int STEPS_BLOCKS = 4;  // blocks an SM (128 registers a thread: no spills)
+constexpr int STEPS_THREADS = 128;
+constexpr int STEPS_A_LAUNCH = 32;  // (a bound on a launch: half a millisecond)
+
+struct StepsArgs {
+    FrontArgs F;
+    RowTables T;
+    PhysDev ph;
+    MapDev map;
+    RowMasks M;
+    float4* rho4S;
+    float4* accS;
+    float4* pos;
+    float4* vel;
+    int collide;
+    int steps;
+};
+
+template <bool KAHAN, bool TENSION>
+__global__ void __launch_bounds__(STEPS_THREADS, STEPS_BLOCKS) k_steps(StepsArgs A) {
+    const FrontArgs& F = A.F;
+    unsigned int round = 0;
+    bool ok = !(*(volatile unsigned int*)F.status & STATUS_DEVICE_WAIT);
+    auto barrier = [&]() { ok = grid_barrier(F.sb.front, ++round, F.waitLimit, F.status); };
+    const int stride = gridDim.x * STEPS_THREADS;
+    const int first = blockIdx.x * STEPS_THREADS + threadIdx.x;
+    for (int s = 0; s < A.steps && ok; s++) {
+        front_phases<false, false, STEPS_THREADS, true>(F, round, ok);
+        if (!ok) break;
+        barrier();
+        if (!ok) break;
+        for (int i = first; i < F.n; i += stride)
+            density_list_one<KAHAN, false, true>(i, F.n, F.posS, F.velS, A.T, F.g, A.ph, A.map, A.rho4S, F.L, A.M);
+        barrier();
+        if (!ok) break;
+        for (int base = blockIdx.x * STEPS_THREADS; base < F.n; base += stride)
+            force_list_one<KAHAN, TENSION, false, true>(base + (int)threadIdx.x, F.n, F.posS, F.velS, A.rho4S,
+                                                        F.sb.workIds, A.ph, A.map, A.collide, F.L, A.M, A.pos, A.vel,
+                                                        A.accS, nullptr);
+        if (s + 1 < A.steps) barrier();
+    }
+    front_leave<STEPS_THREADS>(F);
 }
 
 // ---------------------------------------------------------------------------
@@ -1184,7 +1284,7 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
             ForceTotals<KAHAN, TENSION> A;
             FeatSums fs;
             if (LISTS) {
-                list_rows<TENSION>(
+                list_rows<TENSION, false>(
                     i, F.n, 0, L, F.M, F.posS, F.velS,
                     [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
                         const Pair p(ph, xi, vi, xj, vj);
@@ -1516,6 +1616,35 @@ void launch_force_lists(int n, const float4* posS, const float4* velS, const flo
     }
 #undef SPH_FORCE_LISTS_B
 #undef SPH_FORCE_LISTS
+}
+
+template <bool KAHAN, bool TENSION>
+static void steps_launch(StepsArgs& A, cudaStream_t s) {
+    const int want = std::max((A.F.n + STEPS_THREADS - 1) / STEPS_THREADS, A.F.g.numCells / (16 * STEPS_THREADS));
+    const int grid = std::min(want, resident_blocks<k_steps<KAHAN, TENSION>>(STEPS_THREADS, STEPS_BLOCKS));
+    void* args[] = {&A};
+    cudaLaunchCooperativeKernel((const void*)k_steps<KAHAN, TENSION>, dim3(grid), dim3(STEPS_THREADS), args, 0, s);
+}
+
+bool takes_whole_steps(int n, int numCells) { return n <= STEPS_PARTICLES && numCells <= STEPS_CELLS; }
+
+void launch_steps(int n, float4* pos, float4* vel, GridDev g, SortBuffers sb, RowTables T, float4* posS, float4* velS,
+                  float4* rho4S, float4* accS, PhysDev ph, MapDev map, int collide, const NeighbourLists& L, RowMasks M,
+                  const StepConfig& cfg, int steps, unsigned int* status, cudaStream_t s) {
+    if (n <= 0) return;
+    StepsArgs A{FrontArgs{n, pos, vel, g, sb, posS, velS, status, L, 1, FRONT_ALL, scan_wait_limit()},
+                T, ph, map, M, rho4S, accS, pos, vel, collide, 0};
+    const bool tension = ph.tension != 0.0f;
+    for (; steps > 0; steps -= A.steps) {
+        A.steps = std::min(steps, STEPS_A_LAUNCH);
+        if (cfg.kahan) {
+            if (tension) steps_launch<true, true>(A, s);
+            else steps_launch<true, false>(A, s);
+        } else {
+            if (tension) steps_launch<false, true>(A, s);
+            else steps_launch<false, false>(A, s);
+        }
+    }
 }
 
 }  // namespace sph
