@@ -172,7 +172,7 @@ void free_all(sph_sim* s) {
     for (cudaEvent_t e : s->events) cudaEventDestroy(e);
     void* ptrs[] = {s->pos, s->vel, s->posS, s->velS, s->rho4S, s->accS, s->sb.cnt, s->sb.cellOffset,
                     s->sb.keySlot, s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds,
-                    s->sb.halfOffset, s->sb.front, s->scanBlock,
+                    s->sb.halfOffset, s->sb.front,
                     s->status, s->staging, s->map4, s->mapDist, s->rowStart, s->rowMask, s->diagBuf,
                     s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.posB,
                     s->vl.flags, s->vl.slotScene};
@@ -182,8 +182,7 @@ void free_all(sph_sim* s) {
                       s->ts.splitIds,  s->ts.boundaryIds, s->ts.defaultIds,  s->ts.subIds,
                       s->ts.subPos,    s->ts.subVel,      s->ts.subAcc,      s->ts.subRho,
                       s->ts.subCnt,    s->ts.subOffset,   s->ts.subKeySlot,  s->ts.subTmp,
-                      s->ts.subSortedHash, s->ts.subSortedIds, s->ts.subPosS, s->ts.subVelS, s->ts.markList,
-                      s->subScanBlock};
+                      s->ts.subSortedHash, s->ts.subSortedIds, s->ts.subPosS, s->ts.subVelS, s->ts.markList};
     for (void* p : tsPtrs)
         if (p) cudaFree(p);
     if (s->statusHost) cudaFreeHost(s->statusHost);
@@ -226,7 +225,6 @@ sph_status ensure_two_scale(sph_sim* s) {
     const size_t n4 = (n + 3) & ~(size_t)3;
     const size_t nb = (n + 1023) / 1024;
     const size_t Cs = (size_t)s->P.gridDimSubParticles[0] * s->P.gridDimSubParticles[1] * s->P.gridDimSubParticles[2];
-    const size_t tiles = (Cs + 1 + SCAN_TILE - 1) / SCAN_TILE;
     TwoScaleDev& T = s->ts;
     SPH_CUDA(dalloc(&T.state, n4));
     SPH_CUDA(dalloc(&T.blockCounts, 3 * nb));
@@ -248,7 +246,6 @@ sph_status ensure_two_scale(sph_sim* s) {
     SPH_CUDA(dalloc(&T.subSortedIds, 8 * n));
     SPH_CUDA(dalloc(&T.subPosS, 8 * n));
     SPH_CUDA(dalloc(&T.subVelS, 8 * n));
-    SPH_CUDA(dalloc(&s->subScanBlock, tiles + 2));
     cudaStream_t q = s->stream;
     // index buffers start valid (0): an entry a failed step leaves unwritten
     // still names a child slot or a fine cell
@@ -269,9 +266,7 @@ sph_status ensure_two_scale(sph_sim* s) {
     T.childMode = s->O.childMode;
     s->subSb.cnt = T.subCnt;
     s->subSb.cellOffset = T.subOffset;
-    s->subSb.tileCounter = reinterpret_cast<unsigned int*>(s->subScanBlock);
-    s->subSb.scanFlags = s->subScanBlock + 2;
-    s->subSb.maxTiles = (int)tiles;
+    s->subSb.front = s->sb.front;
     SPH_CUDA(cudaStreamSynchronize(q));
     s->tsReady = true;
     return SPH_OK;
@@ -504,7 +499,6 @@ void enqueue_step(sph_sim* s, int mode, bool timing, bool lists) {
 sph_status alloc_handle(sph_sim* s, int n, long long C) {
     s->n = n;
     s->numCellsTotal = C;
-    const long long tiles = (C + 1 + SCAN_TILE - 1) / SCAN_TILE;
     SPH_CUDA(cudaGetDevice(&s->device));
     SPH_CUDA(cudaStreamCreateWithFlags(&s->ownStream, cudaStreamNonBlocking));
     s->stream = s->ownStream;
@@ -529,10 +523,6 @@ sph_status alloc_handle(sph_sim* s, int n, long long C) {
     // still names a particle or a cell of the handle
     for (int* p : {s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds})
         SPH_CUDA(cudaMemsetAsync(p, 0, sizeof(int) * (size_t)n, s->stream));
-    SPH_CUDA(dalloc(&s->scanBlock, (size_t)tiles + 2));
-    s->sb.tileCounter = reinterpret_cast<unsigned int*>(s->scanBlock);
-    s->sb.scanFlags = s->scanBlock + 2;
-    s->sb.maxTiles = (int)tiles;
     SPH_CUDA(dalloc(&s->sb.front, FRONT_WORDS));
     SPH_CUDA(cudaMemsetAsync(s->sb.front, 0, sizeof(unsigned int) * FRONT_WORDS, s->stream));
     SPH_CUDA(dalloc(&s->status, 1));

@@ -81,10 +81,7 @@ struct SortBuffers {
     int* sortedIds;           // [n]   the reference's permutation (cell, id)
     int* workIds;             // [n]   the working order (cell, x, id) of the sorted arrays
     int* halfOffset;          // [C+1] first working index of each cell's upper x-half
-    unsigned long long* scanFlags;  // decoupled look-back tile states
-    unsigned int* tileCounter;
-    int maxTiles;
-    unsigned int* front;      // [FRONT_WORDS] k_front's barrier and block sums, zero between launches
+    unsigned int* front;      // [FRONT_WORDS] a cooperative launch's barrier and block sums, zero between launches
     const SceneDev* scenes;   // batched handles: per-scene grids (else NULL)
     const int* skip;          // when non-NULL and set on the device, the sorted copies and
                               // tables already hold the current state: the sort stages return
@@ -225,9 +222,8 @@ inline int device_sms() {
     return sms > 0 ? sms : 1;
 }
 
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 32;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+// The cell tables are padded: the scan reads and writes whole vectors.
+constexpr int SCAN_TILE = 8192;
 
 // ---------------------------------------------------------------------------
 // Launch wrappers (sph_kernels.cu)
@@ -257,8 +253,6 @@ bool takes_whole_steps(int n, int numCells);
 void launch_steps(int n, float4* pos, float4* vel, GridDev g, SortBuffers sb, RowTables T, float4* posS, float4* velS,
                   float4* rho4S, float4* accS, PhysDev ph, MapDev map, int collide, const NeighbourLists& L, RowMasks M,
                   const StepConfig& cfg, int steps, unsigned int* status, cudaStream_t s);
-// The fine level's cell offsets (two-scale pass).
-void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s);
 // The cell tables of the sorted copies' positions (sortedHash, sortedIds,
 // cellOffset) after a step that skipped them; the working order, the sorted
 // copies and the lists stay as they are.  `scratch`: n float4.

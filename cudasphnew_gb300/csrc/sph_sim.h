@@ -68,7 +68,6 @@ struct sph_sim {
     int* rowStart = nullptr;          // [9][n] neighbour-row windows recorded by the density stage
     unsigned int* rowMask = nullptr;  // [9][n] their neighbour masks
     sph::SortBuffers sb{};
-    unsigned long long* scanBlock = nullptr;
     unsigned int* status = nullptr;     // device status word
     int* reuse = nullptr;               // device flag: the sorted copies hold the current state
                                         // (set by an accepting audit, used up by the next step)
@@ -105,7 +104,6 @@ struct sph_sim {
     // two-scale pass (allocated on first use)
     sph::TwoScaleDev ts{};
     sph::SortBuffers subSb{};
-    unsigned long long* subScanBlock = nullptr;
     bool tsReady = false;
 
     // CUDA graph of one step of graphMode

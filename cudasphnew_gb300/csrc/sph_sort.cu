@@ -121,170 +121,15 @@ void launch_pack_aos(const float4* in, int n, float* aos, int stride, int offset
         k_pack_aos<<<(n + 255) / 256, 256, 0, s>>>(in, n, aos, stride, offset);
 }
 
-// ---------------------------------------------------------------------------
-// The fine level's scan (two-scale pass): exclusive scan of the C+1 cell
-// counts into cell offsets, one pass with decoupled look-back (Merrill & Garland).  Counts are cleared as they
-// are read, ready for the next step.  Tiles take their index from an atomic
-// counter, so every tile a block waits on has already started; each wait is
-// bounded and latches STATUS_DEVICE_WAIT if it ever gives up.
-// ---------------------------------------------------------------------------
-constexpr unsigned long long FLAG_AGG = 1ull << 32;
-constexpr unsigned long long FLAG_INC = 2ull << 32;
-constexpr int SPIN_LIMIT = 1 << 22;
-
-// `waitLimit` bounds each spin (polls); a negative limit abandons every wait
-// at its first poll (a test of the give-up path: every tile then takes its
-// predecessors as zero).  A tile that gives up latches STATUS_DEVICE_WAIT and
-// completes with a prefix that is a partial sum of the true one, so every
-// offset stays within [0, n] and every index derived from the offsets stays
-// inside its buffer (the step's results are then unspecified and reported).
-__global__ void __launch_bounds__(SCAN_THREADS)
-k_cell_scan(int total, int* __restrict__ cnt, int* __restrict__ out, unsigned long long* flags,
-            unsigned int* tileCounter, unsigned int* status, int waitLimit) {
-    __shared__ int s_tile;
-    __shared__ int s_warp[SCAN_THREADS / 32];
-    __shared__ int s_prefix;
-    if (threadIdx.x == 0) s_tile = (int)atomicAdd(tileCounter, 1u);
-    __syncthreads();
-    const int tile = s_tile;
-    const int base = tile * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-    int v[SCAN_ITEMS];
-    static_assert(SCAN_ITEMS % 4 == 0, "vector loads of four counters");
-    if (base + SCAN_ITEMS <= total) {
-#pragma unroll
-        for (int c = 0; c < SCAN_ITEMS / 4; c++) {
-            const int4 a = *reinterpret_cast<const int4*>(cnt + base + 4 * c);
-            v[4 * c] = a.x;
-            v[4 * c + 1] = a.y;
-            v[4 * c + 2] = a.z;
-            v[4 * c + 3] = a.w;
-            *reinterpret_cast<int4*>(cnt + base + 4 * c) = make_int4(0, 0, 0, 0);
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; k++) {
-            int idx = base + k;
-            v[k] = idx < total ? cnt[idx] : 0;
-            if (idx < total) cnt[idx] = 0;
-        }
-    }
-    int local = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) local += v[k];
-    // block-wide exclusive scan of `local`
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < SCAN_THREADS / 32 ? s_warp[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += t;
-        }
-        if (lane < SCAN_THREADS / 32) s_warp[lane] = w;  // inclusive warp totals
-    }
-    __syncthreads();
-    const int warpExcl = warp > 0 ? s_warp[warp - 1] : 0;
-    const int aggregate = s_warp[SCAN_THREADS / 32 - 1];
-    int excl = warpExcl + incl - local;
-
-    // publish + look back (warp 0)
-    if (warp == 0) {
-        cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> mine(flags[tile]);
-        if (lane == 0) {
-            mine.store((tile == 0 ? FLAG_INC : FLAG_AGG) | (unsigned int)aggregate,
-                       cuda::memory_order_release);
-        }
-        int prefix = 0;
-        if (tile > 0) {
-            int look = tile - 1;
-            bool done = false;
-            while (!done) {
-                int t = look - lane;
-                unsigned long long f = FLAG_INC;  // below tile 0: neutral, inclusive
-                if (t >= 0) {
-                    cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> other(flags[t]);
-                    int spins = 0;
-                    f = other.load(cuda::memory_order_acquire);
-                    if (waitLimit < 0) {
-                        atomicOr(status, STATUS_DEVICE_WAIT);
-                        f = FLAG_INC;  // the wait abandoned at once
-                    }
-                    while ((f >> 32) == 0ull) {
-                        if (++spins > waitLimit) {
-                            atomicOr(status, STATUS_DEVICE_WAIT);
-                            f = FLAG_INC;  // give up: treat as zero, result flagged
-                            break;
-                        }
-                        __nanosleep(32);
-                        f = other.load(cuda::memory_order_acquire);
-                    }
-                    if (t < 0) f = FLAG_INC;
-                }
-                unsigned int incMask = __ballot_sync(0xffffffffu, (f >> 32) == 2ull);
-                int val = (int)(unsigned int)(f & 0xffffffffull);
-                int first = incMask ? __ffs(incMask) - 1 : 32;  // nearest inclusive
-                int contrib = lane <= first ? val : 0;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-                prefix += contrib;
-                if (incMask) done = true;
-                look -= 32;
-            }
-            if (lane == 0)
-                mine.store(FLAG_INC | (unsigned int)(prefix + aggregate), cuda::memory_order_release);
-        }
-        if (lane == 0) s_prefix = prefix;
-    }
-    __syncthreads();
-    int run = s_prefix + excl;
-    if (base + SCAN_ITEMS <= total) {
-#pragma unroll
-        for (int c = 0; c < SCAN_ITEMS / 4; c++) {
-            int4 o;
-            o.x = run;
-            run += v[4 * c];
-            o.y = run;
-            run += v[4 * c + 1];
-            o.z = run;
-            run += v[4 * c + 2];
-            o.w = run;
-            run += v[4 * c + 3];
-            *reinterpret_cast<int4*>(out + base + 4 * c) = o;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; k++) {
-            if (base + k < total) out[base + k] = run;
-            run += v[k];
-        }
-    }
-}
-
 // The poll limit of a wait: SPIN_LIMIT, or the integer in the environment
 // variable SPH_SCAN_WAIT_LIMIT (read at each launch; a captured step graph
 // keeps the value it was captured with).  Tests set it to exercise the
 // give-up path; -1 abandons every wait at once.
 int scan_wait_limit() {
+    constexpr int SPIN_LIMIT = 1 << 22;
     const char* e = getenv("SPH_SCAN_WAIT_LIMIT");
     if (!e || !*e) return SPIN_LIMIT;
     return (int)strtol(e, nullptr, 10);
-}
-
-void launch_cell_scan(int numCells, SortBuffers sb, unsigned int* status, cudaStream_t s) {
-    int total = numCells + 1;
-    int tiles = (total + SCAN_TILE - 1) / SCAN_TILE;
-    // tile counter (first 16 bytes) and the tile states that follow it
-    cudaMemsetAsync(sb.tileCounter, 0, 16 + sizeof(unsigned long long) * (size_t)tiles, s);
-    k_cell_scan<<<tiles, SCAN_THREADS, 0, s>>>(total, sb.cnt, sb.cellOffset, sb.scanFlags, sb.tileCounter, status,
-                                               scan_wait_limit());
 }
 
 // ---------------------------------------------------------------------------
