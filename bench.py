@@ -45,7 +45,7 @@ FORCE_FLOP_PER_PAIR = 40
 # The source files the neighbour kernels are compiled from: a DRAM traffic
 # figure recorded under profiles/ holds only while their hash is unchanged.
 KERNEL_SOURCES = ["cudasphnew_gb300/csrc/" + f for f in
-                  ("sph_step.cu", "sph_device.cuh", "sph_internal.h", "sph_mlp_tile.cuh", "sph_corrector.h",
+                  ("sph_step.cu", "sph_front.cuh", "sph_device.cuh", "sph_internal.h", "sph_mlp_tile.cuh", "sph_corrector.h",
                    "sph_tc.cuh")] + ["include/sph.h"]
 
 
@@ -270,6 +270,10 @@ def cpu_model():
 def fp32_peak(sms, max_mhz):
     """Nominal FP32 rate: SMs x 128 lanes x 2 (FMA) x clock, flop/s."""
     return sms * 128 * 2 * max_mhz * 1e6
+
+
+# kernels of a plain step: front, density, force
+STEP_LAUNCHES = 3
 
 
 def kernel_roofline(kernel, n, C, g3, pairs, t_s, hbm_gbs, fp32, traffic=None):
@@ -749,7 +753,7 @@ def batched_leg(lib, torch, stream, steps=200, peaks=None):
     scs = scenes.config4()
     n = sum(sc.n for sc in scs)
     lists = float(scs[0].options.neighbourSkin) > 0
-    launches = 8 if lists else 6  # with the lists: the decision kernel and the two density forms
+    launches = STEP_LAUNCHES
     roofs = None
     with lib.ParticleSimulation.batch(scs, scs[0].options) as sim:
         sim.set_stream(stream.cuda_stream)
@@ -805,7 +809,9 @@ def batched_leg(lib, torch, stream, steps=200, peaks=None):
             "launches_per_step": launches, "graph": "one CUDA graph launch per step", "tuning": tuning,
             "neighbour_lists": "reused, one build decision per scene" if lists else "per-step search",
             "separate_handles": {"value": n * k / (ms_sep / 1e3), "ms_per_step": ms_sep / k, "steps": k,
-                                 "launches_per_step": launches * len(scs)},
+                                 # (a small handle with lists takes its step in one launch)
+                                 "launches_per_step": sum(1 if lists and len(sc.positions) <= 24576 else launches
+                                                          for sc in scs)},
             "l2": "no flush: working set of the 4.4M-particle batch far exceeds L2", **(roofs or {})}
 
 
@@ -1022,7 +1028,7 @@ def run_ours(args):
                             f"> {L2_BYTES / 2**20:.0f} MiB L2",
                       "graph": "one CUDA graph launch per step", "tuning": tuning},
            "clocks": clk,
-           "gpu_launches": (8 if float(sc.options.neighbourSkin) > 0 else 6) * args.steps,
+           "gpu_launches": STEP_LAUNCHES * args.steps,
            "neighbour_lists": {"skin": float(sc.options.neighbourSkin), "builds_in_timed_region": builds_timed,
                                "note": "the neighbour candidates within (1 + skin) h are rebuilt when a "
                                        "particle has moved 0.45 skin h since the last build; a step that "

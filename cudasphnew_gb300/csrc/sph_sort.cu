@@ -10,8 +10,9 @@
 //   cnt, cellOffset    int[C+1]   per-cell counts / their exclusive scan
 // The sort is a counting sort: every particle takes an arrival slot in its
 // cell with one atomic, a scan turns counts into cell offsets, and a rank pass
-// orders each cell's members by particle id.  The result is the permutation of a stable sort by hash -- the order
-// thrust::sort_by_key produces in the reference (particle_simulation.cu:2340).
+// orders each cell's members by particle id.  The result is the permutation of
+// a stable sort by hash -- the order thrust::sort_by_key produces in the
+// reference (particle_simulation.cu:2340).
 #include <algorithm>
 #include <cstdlib>
 

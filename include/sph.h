@@ -111,7 +111,10 @@ typedef struct sph_options {
                             that builds no lists skips the hash, sort and cell
                             tables (sph_read_cells builds that step's tables
                             when asked, bit exact); only the order in which the
-                            neighbour sums are taken follows the lists.  0: the
+                            neighbour sums are taken follows the lists.  Lists
+                            are not built where the step before, by its own
+                            motion, has outrun those just built: such a step
+                            searches as with 0, until the motion slows.  0: the
                             neighbour search runs in every step, as the
                             reference does (compute_particle_density_pressure,
                             :196-256).  In [0, 0.4].  No reference counterpart. */
@@ -275,7 +278,9 @@ sph_status sph_set_stream(sph_handle h, void* stream);
  * does, with its counts kept on the device. */
 sph_status sph_step(sph_handle h, int mode);
 
-/* Enqueues `count` steps of `mode` (one CUDA-graph launch each once captured). */
+/* Enqueues `count` steps of `mode` (one CUDA-graph launch each once captured;
+ * plain steps of a handle with reused lists and at most 24,576 particles: up
+ * to 32 in one launch).  The results are those of `count` calls of sph_step. */
 sph_status sph_step_many(sph_handle h, int mode, int count);
 
 /* Waits for the handle's stream; returns the latched device status. */
@@ -569,7 +574,8 @@ sph_status sph_time_kernel(sph_handle h, int stage, int reps, float* microsecond
 
 /* How many times the handle's plain and learned steps have built their
  * reused neighbour lists (sph_options.neighbourSkin; 0 when the handle has
- * none; a batch: its scenes' builds summed).  Waits for the handle's stream.
+ * none; a batch: its scenes' builds summed; a step that searches in place of
+ * building is not counted).  Waits for the handle's stream.
  * No reference counterpart. */
 sph_status sph_neighbour_builds(sph_handle h, unsigned int* builds);
 
