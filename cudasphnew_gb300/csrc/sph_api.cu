@@ -306,7 +306,9 @@ sph_status alloc_lists(sph_sim* s) {
     SPH_CUDA(dalloc(&s->vl.flags, (size_t)VL_FLAGS * S + VL_GLOBAL));
     SPH_CUDA(cudaMemsetAsync(s->vl.flags, 0, sizeof(unsigned int) * (VL_FLAGS * S + VL_GLOBAL), s->stream));
     s->vl.numScenes = S;
-    if (S > 1) {  // each sorted slot's scene: scene k fills slots [sceneStart[k], sceneStart[k + 1])
+    // each sorted slot's scene: scene k fills slots [sceneStart[k], sceneStart[k + 1])
+    // (a batch of one scene too: its kernels are the batched forms)
+    if (!s->sceneStart.empty()) {
         std::vector<int> scene(n);
         for (int k = 0; k < S; k++)
             std::fill(scene.begin() + s->sceneStart[(size_t)k], scene.begin() + s->sceneStart[(size_t)k + 1], k);
