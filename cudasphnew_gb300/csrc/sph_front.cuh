@@ -35,6 +35,15 @@ __device__ __forceinline__ unsigned int ordered_bits(float x) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// Whether a launch of waiting blocks goes on: false while a wait that gave up
+// is still to be reported.  Another block of the launch may be setting the
+// word meanwhile, so one thread reads it for its block: a block whose warps
+// saw it before and after would come apart at its own barriers.
+__device__ __forceinline__ bool block_goes_on(const unsigned int* status) {
+    return !__syncthreads_or(threadIdx.x == 0 &&
+                             (*(volatile const unsigned int*)status & STATUS_DEVICE_WAIT) != 0u);
+}
+
 // Waits until every block of the grid has arrived `round` times.
 __device__ __forceinline__ bool grid_barrier(unsigned int* front, unsigned int round, int waitLimit, unsigned int* status) {
     __shared__ int ok;

@@ -186,7 +186,7 @@ template <bool BATCH, bool REL>
 __global__ void __launch_bounds__(FRONT_THREADS, 3) k_front(FrontArgs A) {
     if (A.sb.skip && *A.sb.skip) return;
     unsigned int round = 0;
-    bool ok = !(*(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT);
+    bool ok = block_goes_on(A.status);
     front_phases<BATCH, REL, FRONT_THREADS, false>(A, round, ok);
     if (round || !ok) front_leave<FRONT_THREADS>(A);
 }

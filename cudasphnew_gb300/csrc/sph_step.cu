@@ -1030,7 +1030,7 @@ template <bool KAHAN, bool TENSION>
 __global__ void __launch_bounds__(STEPS_THREADS, STEPS_BLOCKS) k_steps(StepsArgs A) {
     const FrontArgs& F = A.F;
     unsigned int round = 0;
-    bool ok = !(*(volatile unsigned int*)F.status & STATUS_DEVICE_WAIT);
+    bool ok = block_goes_on(F.status);
     auto barrier = [&]() { ok = grid_barrier(F.sb.front, ++round, F.waitLimit, F.status); };
     const int stride = gridDim.x * STEPS_THREADS;
     const int first = blockIdx.x * STEPS_THREADS + threadIdx.x;

@@ -476,7 +476,7 @@ constexpr int TS_SORT_THREADS = 512;
 
 __global__ void __launch_bounds__(TS_SORT_THREADS) k_ts_sort(FrontArgs A, TwoScaleDev T) {
     unsigned int round = 0;
-    bool ok = !(*(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT);
+    bool ok = block_goes_on(A.status);
     auto barrier = [&]() { ok = grid_barrier(A.sb.front, ++round, A.waitLimit, A.status); };
     const int nSub = T.counts[3];
     const int first = blockIdx.x * TS_SORT_THREADS + threadIdx.x, stride = gridDim.x * TS_SORT_THREADS;
