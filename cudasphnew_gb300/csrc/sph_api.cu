@@ -61,7 +61,7 @@ void* host_device_ptr(const void* p) {
 RowMasks masks_of(const sph_sim* s) { return RowMasks{s->rowStart, s->rowMask}; }
 
 RowTables rows_of(const sph_sim* s) {
-    return RowTables{s->sb.cellOffset, s->sb.halfOffset, s->sb.scenes, s->sb.skip};
+    return RowTables{s->sb.cellOffset, s->sb.halfOffset, s->sb.scenes, s->sb.skip, s->status};
 }
 
 GridDev make_grid(const SimulationParameters& P, bool sub) {
@@ -264,6 +264,7 @@ sph_status ensure_two_scale(sph_sim* s) {
         T.splitMax[a] = s->O.splitMax[a];
     }
     T.childMode = s->O.childMode;
+    T.status = s->status;
     s->subSb.cnt = T.subCnt;
     s->subSb.cellOffset = T.subOffset;
     s->subSb.front = s->sb.front;
@@ -520,9 +521,11 @@ sph_status alloc_handle(sph_sim* s, int n, long long C) {
     SPH_CUDA(dalloc(&s->sb.sortedIds, n));
     SPH_CUDA(dalloc(&s->sb.workIds, n));
     SPH_CUDA(dalloc(&s->sb.halfOffset, (size_t)C + 1 + SCAN_TILE));
-    SPH_CUDA(cudaMemsetAsync(s->sb.halfOffset, 0, sizeof(int) * ((size_t)C + 1), s->stream));
     // index buffers start valid (0): an entry a failed step leaves unwritten
-    // still names a particle or a cell of the handle
+    // still names a particle or a cell of the handle, and every row of the
+    // cell tables is empty until a step has filled them
+    for (int* p : {s->sb.cellOffset, s->sb.halfOffset})
+        SPH_CUDA(cudaMemsetAsync(p, 0, sizeof(int) * ((size_t)C + 1 + SCAN_TILE), s->stream));
     for (int* p : {s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds})
         SPH_CUDA(cudaMemsetAsync(p, 0, sizeof(int) * (size_t)n, s->stream));
     SPH_CUDA(dalloc(&s->sb.front, FRONT_WORDS));

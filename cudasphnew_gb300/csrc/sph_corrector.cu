@@ -235,7 +235,7 @@ void enqueue_audit(sph_sim* s, Corrector* C) {
     cudaMemsetAsync(C->errBits, 0, sizeof(unsigned int), q);
     launch_audit(s->n, C->rhoA, C->rhoB, C->errBits, q);
     launch_audit_select(s->n, C->errBits, C->cfg.densityTolerance, C->lPos, C->lVel, s->pos, s->vel, C->counters,
-                        s->reuse, q);
+                        s->reuse, q, s->status);
 }
 
 void enqueue_kind(sph_sim* s, Corrector* C, int kind) {

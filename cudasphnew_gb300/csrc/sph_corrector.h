@@ -104,7 +104,7 @@ void launch_audit(int n, const float* rhoA, const float* rhoB, unsigned int* err
 // sorted copies, last made from the learned result, then hold the state).
 void launch_audit_select(int n, const unsigned int* errBits, float tol, const float4* srcPos,
                          const float4* srcVel, float4* pos, float4* vel, unsigned int* counters, int* reuse,
-                         cudaStream_t s);
+                         cudaStream_t s, const unsigned int* status = nullptr);
 
 // The learned step's force stage with the MLP fused in (sph_step.cu): the
 // pretested pair loop (the density stage must have recorded the masks), or

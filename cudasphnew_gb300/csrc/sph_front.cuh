@@ -316,10 +316,20 @@ __device__ __forceinline__ void front_leave(const FrontArgs& A) {
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (*(volatile unsigned int*)(front + FRONT_FAILED)) {
-        for (long long c = t; c < (((long long)A.g.numCells + 4) & ~3ll); c += THREADS) A.sb.cnt[c] = 0;
-        if (A.lists)
-            for (int k = t; k < A.L.numScenes; k += THREADS) A.L.flags[VL_BUILD * A.L.numScenes + k] = 1u;
+    const unsigned int failed = *(volatile unsigned int*)(front + FRONT_FAILED);
+    const unsigned int latched = *(volatile unsigned int*)A.status & STATUS_DEVICE_WAIT;
+    if (A.lists && latched)
+        for (int k = t; k < A.L.numScenes; k += THREADS) {
+            A.L.flags[VL_BUILD * A.L.numScenes + k] = 1u;
+            A.L.flags[VL_BUILD_NOW * A.L.numScenes + k] = VL_NOTHING;
+        }
+    if (failed) {
+        // (offsets of two different steps side by side: an empty grid instead)
+        for (long long c = t; c < (((long long)A.g.numCells + 4) & ~3ll); c += THREADS) {
+            A.sb.cnt[c] = 0;
+            A.sb.cellOffset[c] = 0;
+            if (A.sb.halfOffset) A.sb.halfOffset[c] = 0;
+        }
     }
     __syncthreads();
     if (t < FRONT_SUMS) front[t] = 0u;

@@ -113,6 +113,7 @@ struct TwoScaleDev {
     float4* subVelS;            // [8n] child velocities in that order
     float splitMin[3], splitMax[3];
     int childMode;              // sph_options.childMode
+    const unsigned int* status; // as RowTables::status
 };
 
 // Per-row lookup tables of the neighbour search.
@@ -121,6 +122,8 @@ struct RowTables {
     const int* halfOffset;  // [C+1]
     const SceneDev* scenes; // batched handles: per-scene grids, constants, maps (else NULL)
     const int* skip;        // as SortBuffers::skip, read by the density stage only
+    const unsigned int* status;  // with STATUS_DEVICE_WAIT latched there is no sorted step to work on
+                                 // (the list kernels know from VL_NOTHING)
 };
 
 // Reused neighbour lists (sph_options.neighbourSkin).  When the lists are
@@ -162,8 +165,9 @@ enum : int {
 // step has moved some particle past the rebuild distance by itself, lists
 // built for it were never used, and the steps that follow search as a handle
 // without lists does (recording windows of radius h) until one stays within
-// the distance again.
-enum : unsigned int { VL_REUSES = 0, VL_BUILDS = 1, VL_SEARCHES = 2 };
+// the distance again.  VL_NOTHING: a wait of the step's sort gave up (or an
+// earlier one's did, still to be reported), and the list kernels do nothing.
+enum : unsigned int { VL_REUSES = 0, VL_BUILDS = 1, VL_SEARCHES = 2, VL_NOTHING = 3 };
 // Two words after the per-scene flags: whether this step sorts (some scene
 // builds; a step that builds nothing keeps the working order and skips the
 // hash, scan and scatter), and whether the cell tables on the device are

@@ -502,7 +502,7 @@ __global__ void k_audit(int n, const float* __restrict__ rhoA, const float* __re
 __global__ void k_audit_select(int n, const unsigned int* __restrict__ errBits, float tol,
                                const float4* __restrict__ srcPos, const float4* __restrict__ srcVel,
                                float4* __restrict__ pos, float4* __restrict__ vel, unsigned int* counters,
-                               int* reuse) {
+                               int* reuse, const unsigned int* __restrict__ status) {
     const unsigned int bits = *errBits;
     const bool accept = __uint_as_float(bits) <= tol;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -511,7 +511,7 @@ __global__ void k_audit_select(int n, const unsigned int* __restrict__ errBits, 
         if (!accept) counters[1] += 1;  // rollbacks
         counters[2] = bits;             // last error
         counters[3] = max(counters[3], bits);
-        if (reuse) *reuse = accept ? 1 : 0;
+        if (reuse) *reuse = accept && !(*status & STATUS_DEVICE_WAIT) ? 1 : 0;  // (sorts that gave up left no copies)
     }
     if (accept && i < n) {
         pos[i] = srcPos[i];
@@ -571,8 +571,9 @@ void launch_audit(int n, const float* rhoA, const float* rhoB, unsigned int* err
 }
 
 void launch_audit_select(int n, const unsigned int* errBits, float tol, const float4* srcPos, const float4* srcVel,
-                         float4* pos, float4* vel, unsigned int* counters, int* reuse, cudaStream_t s) {
-    k_audit_select<<<(n + 255) / 256, 256, 0, s>>>(n, errBits, tol, srcPos, srcVel, pos, vel, counters, reuse);
+                         float4* pos, float4* vel, unsigned int* counters, int* reuse, cudaStream_t s,
+                         const unsigned int* status) {
+    k_audit_select<<<(n + 255) / 256, 256, 0, s>>>(n, errBits, tol, srcPos, srcVel, pos, vel, counters, reuse, status);
 }
 
 }  // namespace sph

@@ -173,11 +173,12 @@ int scan_wait_limit() {
 // reuses its lists has its ids ranked and its state gathered into its kept order.
 //
 // Every wait is bounded.  A block whose wait gives up latches
-// STATUS_DEVICE_WAIT and leaves; the rest follow, and the last to leave clears
-// the counts and asks for new lists: every offset and id left behind is of
-// this step or an earlier one, so every index derived from them stays inside
-// its buffer (the step's results are unspecified and reported).  Until the
-// condition has been reported, further steps sort nothing.
+// STATUS_DEVICE_WAIT and leaves; the rest follow (no block passes the barrier
+// after one that a block has left), and the last to leave empties the counts
+// and the cell tables, whose offsets may be of two steps, and asks for new
+// lists.  Every id left behind is of this step or an earlier one.  The stages
+// that follow find the condition (gave_up, VL_NOTHING) and leave the state as
+// it was, and until it has been reported further steps do nothing.
 // ---------------------------------------------------------------------------
 constexpr int FRONT_THREADS = 512;
 constexpr int FRONT_WIDE = 1 << 19;

@@ -98,8 +98,10 @@ __global__ void __launch_bounds__(256, REL ? 5 : 6)
 k_density(int n, const float4* __restrict__ posS, RowTables T, GridDev g_, PhysDev ph_, MapDev map_, int window,
           float4* __restrict__ rho4S, RowMasks M) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (T.skip && *T.skip)) return;
+    if (i >= n) return;
     const float4 xi = posS[i];
+    const bool off = gave_up(T.status);
+    if ((T.skip && *T.skip) || off) return;
     // batched handles: the particle's own scene supplies grid, constants and maps
     const SceneDev* S = BATCH ? T.scenes + __float_as_int(xi.w) : nullptr;
     const GridDev& g = BATCH ? S->g : g_;
@@ -297,6 +299,7 @@ __device__ __forceinline__ void density_list_one(int i, int n, float4* posS, flo
     const int scene = BATCH ? L.slotScene[i] : 0;
     const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
     if (kind != VL_REUSES) {
+        if (!FRESH && kind == VL_NOTHING) return;
         density_build_one<KAHAN, BATCH, FRESH>(i, n, kind == VL_BUILDS, scene, posS, velS, T, g, ph_, map_, rho4S, L, M);
         return;
     }
@@ -742,6 +745,7 @@ __global__ void __launch_bounds__(256, FEAT ? 3 : (BATCH || TENSION || REL || FO
     const float4 xi = F.posS[i];
     const float4 vi = F.velS[i];
     const float4 ri = F.rho4S[i];
+    if (gave_up(F.T.status)) return;
     const SceneDev* S = BATCH ? F.T.scenes + __float_as_int(xi.w) : nullptr;
     const GridDev& g = BATCH ? S->g : F.g;
     const PhysDev& ph = BATCH ? S->ph : F.ph;
@@ -838,10 +842,10 @@ __global__ void __launch_bounds__(256, FEAT ? 3 : (BATCH || TENSION || REL || FO
 // `tested` when it is known to lie within h), `row` with the sums of each
 // row's, window's or (group true) list group's pairs.
 template <bool TENSION, bool FRESH, class PAIR, class ROW>
-__device__ __forceinline__ void list_rows(int i, int n, int scene, const NeighbourLists& L, const RowMasks& M,
+__device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const NeighbourLists& L, const RowMasks& M,
                                           const float4* posS, const float4* velS,
                                           PAIR&& pair, ROW&& row) {
-    if (L.flags[VL_BUILD_NOW * L.numScenes + scene]) {
+    if (kind != VL_REUSES) {
         int svN = load<FRESH>(M.start + i);
         unsigned int mN = load<FRESH>(M.mask + i);
 #pragma unroll 1
@@ -925,11 +929,13 @@ __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS,
                                                const SceneDev* scenes) {
     float d2 = 0.f;
     int scene = 0;
-    if (i < n) {
+    auto particle = [&]() {
         const float4 xi = posS[i];
         const float4 vi = velS[i];
         const float4 ri = rho4S[i];
         if (BATCH) scene = L.slotScene[i];
+        const unsigned int kind = L.flags[VL_BUILD_NOW * L.numScenes + scene];
+        if (!FRESH && kind == VL_NOTHING) return;
         const PhysDev& ph = BATCH ? scenes[scene].ph : ph_;
         const MapDev& map = BATCH ? scenes[scene].map : map_;
         const float h2 = ph.h2;
@@ -937,7 +943,7 @@ __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS,
         // (a neighbour's p/rho^2 and 1/rho ride in the fourth lanes of its
         // sorted position and velocity, written by the density stage)
         list_rows<TENSION, FRESH>(
-            i, n, scene, L, M, posS, velS,
+            i, n, kind, L, M, posS, velS,
             [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
                 Pair p(ph, xi, vi, xj, vj);
                 const bool in = tested || neighbour_r2(p.r2, h2);
@@ -969,7 +975,8 @@ __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS,
         const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
         d2 = dx * dx + dy * dy + dz * dz;
         if (!(d2 == d2)) d2 = __uint_as_float(0x7f800000u);  // NaN: as far as it gets
-    }
+    };
+    if (i < n) particle();
     record_displacement<BATCH>(L, scene, d2);
 }
 
@@ -1079,6 +1086,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 4) k_force_staged(ForceArgs F, 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4* buf = reinterpret_cast<float4*>(stsm) + warp * (2 * 3 * ST_ROW);  // [buffer][P, V, Q][ST_ROW]
     uint64_t* bars = reinterpret_cast<uint64_t*>(stsm + ST_WARPS * 2 * 3 * ST_ROW * 16) + 2 * warp;
+    // the whole warp leaves or none (others may be latching the word)
+    if (__any_sync(0xffffffffu, *(volatile const unsigned int*)status & STATUS_DEVICE_WAIT)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < F.n;  // no early return: the warp stages its rows together
     if (lane == 0) {
@@ -1261,14 +1270,22 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
     if (t == 0) {
         tc::mbar_init(bar, 1);
         tc::mbar_init(wbar, 1);
-        sOk = 1;
+        // one thread reads the latch for its block (others may be setting it)
+        sOk = *(volatile unsigned int*)status & STATUS_DEVICE_WAIT ? 3 : 1;
         // the weight image arrives by one TMA bulk copy while the pair loop runs
-        tc::mbar_arrive_expect_tx(wbar, IMG_FWD_BYTES);
-        tc::bulk_g2s(sm + L_W, m.image, IMG_FWD_BYTES, wbar);
+        if (sOk == 1) {
+            tc::mbar_arrive_expect_tx(wbar, IMG_FWD_BYTES);
+            tc::bulk_g2s(sm + L_W, m.image, IMG_FWD_BYTES, wbar);
+        }
     }
     if (warp == 0) tc::tmem_alloc(slot, L_TMEM);
     tc::cta_sync();
     const uint32_t tb = *slot;
+    if (sOk == 3) {
+        tc::cta_sync();
+        if (warp == 0) tc::tmem_dealloc(tb, L_TMEM);
+        return;
+    }
     const int i = blockIdx.x * L_THREADS + t;
     const bool valid = i < F.n;
     float3 x = make_float3(0.f, 0.f, 0.f), v = x;
@@ -1285,7 +1302,7 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
             FeatSums fs;
             if (LISTS) {
                 list_rows<TENSION, false>(
-                    i, F.n, 0, L, F.M, F.posS, F.velS,
+                    i, F.n, L.flags[VL_BUILD_NOW * L.numScenes], L, F.M, F.posS, F.velS,
                     [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
                         const Pair p(ph, xi, vi, xj, vj);
                         if (tested || neighbour_r2(p.r2, ph.h2)) {
@@ -1345,7 +1362,7 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
     unsigned char* myH = sm + L_H + half * 16384;
     const uint32_t tl = tc::tmem_at(tb, 32 * (warp & 3), 64 * half);  // this warp's lanes of its tile
     uint32_t phase = 0;
-    // sOk: 1 running, 0 an MMA wait gave up, 2 the weight copy never landed
+    // sOk: 1 running, 0 an MMA wait gave up, 2 the weight copy never landed (3, above: a wait of the sort gave up)
     if (t == 0 && !tc::mbar_wait(wbar, 0, WAIT_LIMIT)) {
         sOk = 2;
         atomicOr(status, STATUS_DEVICE_WAIT);

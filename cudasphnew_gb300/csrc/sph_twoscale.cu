@@ -179,6 +179,7 @@ __device__ __forceinline__ float group_total(float v) {
 // Also lists the split particles' working-order indices for the marking
 // (warp-aggregated appends, in no fixed order: the marks do not depend on it).
 __global__ void k_ts_state(int n, const float4* __restrict__ posS, const int* __restrict__ workIds, TwoScaleDev T) {
+    if (gave_up(T.status)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool split = false;
@@ -364,7 +365,7 @@ __global__ void k_ts_children(int n, float4* __restrict__ posS, float4* __restri
                               const int* __restrict__ workIds, float mass, PhysDev ph, int collideFlag,
                               float4* __restrict__ pos, float4* __restrict__ vel, TwoScaleDev T) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+    if (k >= n || gave_up(T.status)) return;
     const int id = workIds[k];
     const unsigned int code = T.state[id] & 15u;
     const int was = state_class(code >> 2), now = state_class(code & 3u);
@@ -421,6 +422,7 @@ __global__ void __launch_bounds__(TS_WARP_BLOCK) k_ts_project(const float4* __re
                                                               const float4* __restrict__ rho4S,
                                                               const int* __restrict__ cellOffset, GridDev g,
                                                               float hs, TwoScaleDev T) {
+    if (gave_up(T.status)) return;
     const int first = 8 * T.counts[0];
     const int nSub = T.counts[3];
     const float hs2 = __fmul_rn(hs, hs);
@@ -515,6 +517,7 @@ __global__ void __launch_bounds__(TS_SORT_THREADS) k_ts_sort(FrontArgs A, TwoSca
 // compute_sub_particle_density_pressure (:259-313) for regular children.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(TS_WARP_BLOCK) k_ts_subdensity(GridDev g, PhysDev ph, TwoScaleDev T) {
+    if (gave_up(T.status)) return;
     const int nReg = 8 * T.counts[0];
     const int lane = threadIdx.x & 31, gl = lane & (TS_G - 1), grp = lane / TS_G;
     const int warps = gridDim.x * (TS_WARP_BLOCK / 32);
@@ -576,6 +579,7 @@ constexpr int TS_QUEUE = TS_G * TS_GBATCH + TS_G;
 
 __global__ void __launch_bounds__(TS_WARP_BLOCK) k_ts_subforce(GridDev g, PhysDev ph, TwoScaleDev T) {
     __shared__ int s_queue[TS_WARP_BLOCK / TS_G][TS_QUEUE];
+    if (gave_up(T.status)) return;
     const int nReg = 8 * T.counts[0];
     const int nSub = T.counts[3];
     for (int idx = nReg + blockIdx.x * TS_WARP_BLOCK + threadIdx.x; idx < nSub; idx += gridDim.x * TS_WARP_BLOCK) {
