@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -46,16 +47,24 @@ sph_status record_error(sph_status st, const char* file, int line, const std::st
 
 namespace sph {
 
-// The device address of page-locked host memory (pinned or registered),
-// which kernels read and write directly over the host link; NULL for
-// pageable memory, which goes through the staging buffer.
-void* host_device_ptr(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();  // pageable memory on older drivers: clear the error
-        return nullptr;
+// The device address of `bytes` (> 0) of page-locked host memory (pinned or
+// registered) that hold floats, which kernels read and write directly over
+// the host link; NULL for memory that is not page-locked from end to end and
+// for floats off their 4-byte boundary, which go through a device buffer.
+void* host_device_ptr(const void* p, size_t bytes) {
+    if (reinterpret_cast<uintptr_t>(p) % alignof(float)) return nullptr;
+    const char* ends[2] = {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1};
+    char* dev[2];
+    for (int k = 0; k < 2; k++) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, ends[k]) != cudaSuccess) {
+            cudaGetLastError();  // pageable memory on older drivers: clear the error
+            return nullptr;
+        }
+        if (a.type != cudaMemoryTypeHost) return nullptr;
+        dev[k] = static_cast<char*>(a.devicePointer);
     }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+    return dev[1] - dev[0] == ends[1] - ends[0] ? dev[0] : nullptr;
 }
 
 RowMasks masks_of(const sph_sim* s) { return RowMasks{s->rowStart, s->rowMask}; }
@@ -918,7 +927,7 @@ sph_status read_two_scale(sph_sim* s, int field, void* dst, size_t bytes) {
         // page-locked memory takes the positions from the kernel itself, over the
         // host link (as read_field; 25 MB in 140 us, 300 through a device buffer
         // allocated for the call)
-        if (float* direct = static_cast<float*>(host_device_ptr(dst))) {
+        if (float* direct = static_cast<float*>(host_device_ptr(dst, need))) {
             launch_pack_aos(s->ts.subPos, (int)(8 * n), direct, 3, 0, q);
             SPH_CUDA(cudaGetLastError());
             SPH_CUDA(cudaStreamSynchronize(q));
@@ -1009,7 +1018,7 @@ static sph_status read_field(sph_sim* s, int field, void* dst, size_t bytes, boo
     // pageable destinations go through the staging buffer and one DMA copy
     float* direct = nullptr;
     if (wait && ((field == SPH_FIELD_VERTEX_DATA && !s->O.cellRelative) || field == SPH_FIELD_VELOCITY))
-        direct = static_cast<float*>(host_device_ptr(dst));
+        direct = static_cast<float*>(host_device_ptr(dst, need));
     float* out = direct ? direct : s->staging;
     if (!wait) {
         // packed on the handle's stream into a buffer of its own, copied to
@@ -1098,7 +1107,7 @@ sph_status sph_write(sph_handle s, int field, const void* src, size_t bytes) {
         case SPH_FIELD_VELOCITY: {
             if (bytes < sizeof(float) * 3 * (size_t)n) SPH_FAIL(SPH_ERR_INVALID_ARGUMENT, "source too small");
             // page-locked sources are read by the unpacking kernel itself
-            const float* in = static_cast<const float*>(host_device_ptr(src));
+            const float* in = static_cast<const float*>(host_device_ptr(src, sizeof(float) * 3 * (size_t)n));
             float4* target = field == SPH_FIELD_VERTEX_DATA ? s->pos : s->vel;
             if (!in) {
                 SPH_CUDA(cudaMemcpyAsync(s->staging, src, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, q));

@@ -188,8 +188,9 @@ void corrector_free(sph_sim* s);
 sph_status latched_status(sph_sim* s);
 // The status held in statusHost (already copied back and synchronised).
 sph_status status_of_host_copy(const sph_sim* s);
-// Device address of page-locked host memory, or NULL (pageable memory).
-void* host_device_ptr(const void* p);
+// Device address of floats in page-locked host memory, or NULL (pageable, in
+// part pageable, off a 4-byte boundary).
+void* host_device_ptr(const void* p, size_t bytes);
 // Allocates the device state of n particles over C cells (zeroed counters,
 // velocities and per-step outputs) and the handle's stream.
 sph_status alloc_handle(sph_sim* s, int n, long long C);
