@@ -191,9 +191,15 @@ __device__ float eval_viscosity_kernel(const MapArgs& A, float sqDist) {
     const float x = A.h - dist;
     if (A.viscosityHi == 0.0f) return (float)(A.viscosityCoeff * x);
     // the FP64 product rounded to FP32, from FP32 operations (the FP64 pipe and
-    // its conversions held the sums: 315 -> 125 us for a 128^3 map)
+    // its conversions held the sums: 315 -> 125 us for a 128^3 map).  The two
+    // products are within 2^-46 of the exact one, the FP64 product within
+    // 2^-53: where all numbers within 2^-44 of theirs round alike, so does it.
     const float p = A.viscosityHi * x;
-    return p + __fmaf_rn(A.viscosityLo, x, __fmaf_rn(A.viscosityHi, x, -p));
+    const float low = __fmaf_rn(A.viscosityLo, x, __fmaf_rn(A.viscosityHi, x, -p));
+    const float s = p + low;
+    const float rest = low - (s - p), slack = s * 5.6843419e-14f;
+    if (s + (rest - slack) == s && s + (rest + slack) == s) return s;
+    return (float)(A.viscosityCoeff * x);
 }
 
 __device__ void node_pos(const MapArgs& A, int i, int j, int k, float* p) {
