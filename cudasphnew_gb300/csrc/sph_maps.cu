@@ -173,7 +173,8 @@ __device__ float solid_estimate(const MapArgs& A, const float* x, float& margin)
         for (int k = 0; k < 6; k++) scale += fabsf(S.p[k]);
         s = fminf(s, d);
     }
-    margin = 128.0f / 16777216.0f * scale;
+    // (lengths whose squares leave FP32's range have no estimate either)
+    margin = scale > 1e-15f && scale < 1e15f ? 128.0f / 16777216.0f * scale : INFINITY;
     return s;
 }
 
