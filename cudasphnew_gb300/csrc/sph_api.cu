@@ -842,6 +842,10 @@ sph_status sph_step_many(sph_handle s, int mode, int count) {
         return SPH_OK;
     }
     if (mode == SPH_STEP_PLAIN && whole_steps(s)) {
+        // (refused on a stream that is being captured, as the step graph of the other handles is)
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        SPH_CUDA(cudaStreamIsCapturing(s->stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) SPH_FAIL(SPH_ERR_CUDA, cudaGetErrorString(cudaErrorIllegalState));
         enqueue_whole_steps(s, count);
         SPH_CUDA(cudaGetLastError());
         s->numTimeSteps += (unsigned int)count;
