@@ -187,7 +187,7 @@ __device__ __forceinline__ void front_rank(const FrontArgs& A) {
 template <bool BATCH, bool REL, int THREADS, bool FRESH>
 __device__ __forceinline__ void front_phases(const FrontArgs& A, unsigned int& round, bool& ok) {
     __shared__ int warps[THREADS / 32];
-    __shared__ int carry;
+    __shared__ int parts[THREADS / 32];  // each warp's counts, from the sums to the scan
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     unsigned int* front = A.sb.front;
     unsigned int* f = A.L.flags;
@@ -224,55 +224,69 @@ __device__ __forceinline__ void front_phases(const FrontArgs& A, unsigned int& r
         front_hash<BATCH, REL, THREADS>(A);
         if (A.phases & FRONT_SCAN) barrier();
     }
-    // this block's stretch of cells, four at a time (the buffers are padded)
-    const long long total = ((long long)A.g.numCells + 4) & ~3ll;  // numCells + 1 counts
-    const long long per = ((total / 4 + gridDim.x - 1) / gridDim.x) * 4;
-    const long long c0 = per * blockIdx.x, c1 = min(c0 + per, total);
+    // This block's stretch of cells and this warp's part of it, in vectors of
+    // four counts (numCells + 1 of them; the buffers are padded).  A warp scans
+    // its part on its own, SCAN_UNROLL vectors a lane in flight: few particles
+    // in a grid of many cells (4,096 in 13.8 million) are a step of 91 us so, 353 when
+    // every 2,048 cells took the block three barriers.
+    constexpr int WARPS = THREADS / 32, SCAN_UNROLL = 2;
+    const int4* cnt = reinterpret_cast<const int4*>(A.sb.cnt);
+    const long long quads = ((long long)A.g.numCells + 4) / 4;
+    const long long blockQuads = (quads + gridDim.x - 1) / gridDim.x, warpQuads = (blockQuads + WARPS - 1) / WARPS;
+    const long long blockEnd = min(blockQuads * (blockIdx.x + 1), quads);
+    const long long q0 = min(blockQuads * blockIdx.x + warpQuads * warp, blockEnd), q1 = min(q0 + warpQuads, blockEnd);
     if (ok && (A.phases & FRONT_SUM)) {
         int sum = 0;
-        for (long long c = c0 + 4 * t; c < c1; c += 4 * THREADS) {
-            const int4 v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
+#pragma unroll 4
+        for (long long q = q0 + lane; q < q1; q += 32) {
+            const int4 v = cnt[q];
             sum += v.x + v.y + v.z + v.w;
         }
-        sum = front_block_sum<THREADS>(sum, warps);
-        if (t == 0) front[FRONT_SUMS + blockIdx.x] = (unsigned int)sum;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) parts[warp] = sum;
+        __syncthreads();
+        if (t == 0) {
+            int all = 0;
+            for (int w = 0; w < WARPS; w++) all += parts[w];
+            front[FRONT_SUMS + blockIdx.x] = (unsigned int)all;
+        }
         barrier();
     }
     if (ok && (A.phases & FRONT_SCAN)) {
-        int before = 0;
-        for (int b = t; b < (int)blockIdx.x; b += THREADS) before += (int)front[FRONT_SUMS + b];
-        before = front_block_sum<THREADS>(before, warps);
-        for (long long base = c0; base < c1; base += 4 * THREADS) {
-            const long long c = base + 4 * t;
-            int4 v = make_int4(0, 0, 0, 0);
-            if (c < c1) {
-                v = *reinterpret_cast<const int4*>(A.sb.cnt + c);
-                *reinterpret_cast<int4*>(A.sb.cnt + c) = make_int4(0, 0, 0, 0);
-            }
-            const int local = v.x + v.y + v.z + v.w;
-            int incl = local;
+        int run = 0;
+        for (int b = t; b < (int)blockIdx.x; b += THREADS) run += (int)front[FRONT_SUMS + b];
+        run = front_block_sum<THREADS>(run, warps);
+        for (int w = 0; w < warp; w++) run += parts[w];
+        for (long long base = q0; base < q1; base += 32 * SCAN_UNROLL) {
+            int4 v[SCAN_UNROLL];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += u;
+            for (int u = 0; u < SCAN_UNROLL; u++) {
+                const long long q = base + 32 * u + lane;
+                v[u] = q < q1 ? cnt[q] : make_int4(0, 0, 0, 0);
             }
-            __syncthreads();  // (the last use of `warps` and `carry`)
-            if (lane == 31) warps[warp] = incl;
-            __syncthreads();
-            int run = before + incl - local;
-            for (int w = 0; w < warp; w++) run += warps[w];
-            if (t == THREADS - 1) carry = run + local;
-            if (c < c1) {
+#pragma unroll
+            for (int u = 0; u < SCAN_UNROLL; u++) {
+                const long long q = base + 32 * u + lane;
+                const int local = v[u].x + v[u].y + v[u].z + v[u].w;
+                int incl = local;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int x = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += x;
+                }
                 int4 o;
-                o.x = run;
-                o.y = o.x + v.x;
-                o.z = o.y + v.y;
-                o.w = o.z + v.z;
-                *reinterpret_cast<int4*>(A.sb.cellOffset + c) = o;
-                if (A.sb.halfOffset) *reinterpret_cast<int4*>(A.sb.halfOffset + c) = o;
+                o.x = run + incl - local;
+                o.y = o.x + v[u].x;
+                o.z = o.y + v[u].y;
+                o.w = o.z + v[u].z;
+                if (q < q1) {
+                    if (local) reinterpret_cast<int4*>(A.sb.cnt)[q] = make_int4(0, 0, 0, 0);
+                    reinterpret_cast<int4*>(A.sb.cellOffset)[q] = o;
+                    if (A.sb.halfOffset) reinterpret_cast<int4*>(A.sb.halfOffset)[q] = o;
+                }
+                run += __shfl_sync(0xffffffffu, incl, 31);
             }
-            __syncthreads();
-            before = carry;
         }
         if (A.phases & FRONT_SCATTER) barrier();
     }
