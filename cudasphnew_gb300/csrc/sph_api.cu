@@ -183,7 +183,7 @@ void free_all(sph_sim* s) {
                     s->sb.keySlot, s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds,
                     s->sb.halfOffset, s->sb.front,
                     s->status, s->staging, s->map4, s->mapDist, s->rowStart, s->rowMask, s->diagBuf,
-                    s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.posB,
+                    s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.masks, s->vl.posB,
                     s->vl.flags, s->vl.slotScene};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -306,11 +306,18 @@ void set_list_radius(sph_sim* s) {
     s->vl.skinFrac = skin;
 }
 
-sph_status alloc_lists(sph_sim* s) {
+double list_candidates(const PhysDev& ph, float skin) {
+    const double R = (1.0 + (double)skin) * (double)ph.h;
+    const double inside = (double)ph.restDensity / (double)ph.mass * 4.18879 * R * R * R;
+    return std::isfinite(inside) ? inside : 0.0;
+}
+
+// (room for twice the candidates of a particle inside the fluid at rest, so
+// that only a fluid compressed to twice its density records windows)
+sph_status alloc_lists(sph_sim* s, double candidates) {
     if (!(s->O.neighbourSkin > 0.0f) || s->O.cellRelative) return SPH_OK;
     const size_t n = (size_t)s->n;
     const int S = std::max(s->numScenes, 1);
-    SPH_CUDA(dalloc(&s->vl.list, VL_GROUPS * n));
     SPH_CUDA(dalloc(&s->vl.groups, n));
     SPH_CUDA(dalloc(&s->vl.posB, n));
     SPH_CUDA(dalloc(&s->vl.flags, (size_t)VL_FLAGS * S + VL_GLOBAL));
@@ -325,6 +332,17 @@ sph_status alloc_lists(sph_sim* s) {
         SPH_CUDA(dalloc(&s->vl.slotScene, n));
         SPH_CUDA(cudaMemcpy(s->vl.slotScene, scene.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     }
+    s->vl.capacity = (int)std::min(std::max(std::ceil(2.0 * candidates / 4.0), (double)VL_GROUPS_MIN),
+                                   (double)VL_GROUPS_MAX);
+    // (where memory is short, fewer groups: more particles record windows)
+    cudaError_t e = dalloc(&s->vl.list, (size_t)s->vl.capacity * n);
+    while (e == cudaErrorMemoryAllocation && s->vl.capacity > VL_GROUPS_SHORT) {
+        cudaGetLastError();
+        s->vl.capacity = std::max(s->vl.capacity / 2, VL_GROUPS_SHORT);
+        e = dalloc(&s->vl.list, (size_t)s->vl.capacity * n);
+    }
+    SPH_CUDA(e);
+    if (s->O.neighbourSkin > VL_MASK_SKIN) SPH_CUDA(dalloc(&s->vl.masks, (size_t)((s->vl.capacity + 7) / 8) * n));
     SPH_CUDA(cudaMemsetAsync(s->vl.groups, 0, n, s->stream));
     launch_list_far_record((int)n, s->posS, s->velS, s->stream);
     set_list_radius(s);
@@ -683,7 +701,7 @@ sph_status sph_create(const SimulationParameters* params, const sph_options* opt
     const int n = (int)params->numParticles;
     const long long C = (long long)params->gridDim[0] * params->gridDim[1] * params->gridDim[2];
     st = alloc_handle(s, n, C);
-    if (!st) st = alloc_lists(s);
+    if (!st) st = alloc_lists(s, list_candidates(make_phys(s->P, s->O), s->O.neighbourSkin));
     if (st) {
         free_all(s);
         delete s;
@@ -1366,7 +1384,7 @@ static sph_status autotune_lists(sph_sim* s, int reps, sph_tuning* chosen) {
                 {s->sb.workIds, nullptr, sizeof(int) * n},      {s->sb.cellOffset, nullptr, sizeof(int) * C1},
                 {s->sb.halfOffset, nullptr, sizeof(int) * C1},
                 {s->vl.flags, nullptr, sizeof(unsigned int) * (VL_FLAGS * s->vl.numScenes + VL_GLOBAL)},
-                {s->vl.list, nullptr, sizeof(int4) * VL_GROUPS * n},
+                {s->vl.list, nullptr, sizeof(int4) * (size_t)s->vl.capacity * n},
                 {s->vl.groups, nullptr, (size_t)n},             {s->vl.posB, nullptr, sizeof(float4) * n}};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto cleanup = [&]() {
@@ -1691,8 +1709,13 @@ sph_status sph_time_kernel(sph_handle s, int stage, int reps, float* microsecond
                          s->status);
         }
     };
-    if (stage == ST_FORCE && !lists)  // the masks of the current tuning
-        launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, s->cfg, st);
+    if (stage == ST_FORCE) {  // the masks of the current tuning, or of the lists
+        if (lists)
+            launch_density_lists(n, s->posS, s->velS, rows_of(s), g, ph, s->map, s->rho4S, s->vl, masks_of(s), s->cfg,
+                                 st);
+        else
+            launch_density(n, s->posS, rows_of(s), g, ph, s->map, s->rho4S, s->rowStart, s->rowMask, s->cfg, st);
+    }
     launch();  // warm
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t e = cudaEventCreate(&e0);

@@ -128,7 +128,9 @@ sph_status sph_create_batch(const sph_scene* scenes, int numScenes, const sph_op
                                q));
     s->sb.scenes = s->scenesDev;
     // reused neighbour lists, one build decision per scene
-    if (sph_status sl = alloc_lists(s)) return bail(sl);
+    double candidates = 0.0;
+    for (const SceneDev& d : table) candidates = std::max(candidates, list_candidates(d.ph, O.neighbourSkin));
+    if (sph_status sl = alloc_lists(s, candidates)) return bail(sl);
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaStreamSynchronize(q));  // `table` leaves scope
 #undef BATCH_CUDA

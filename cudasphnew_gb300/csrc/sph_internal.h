@@ -133,9 +133,13 @@ struct RowTables {
 // with slot n, a record far from everything that the sorted copies keep there).
 // Later steps keep that working order (the state is gathered into it) and
 // visit only those candidates, until some particle has moved farther than
-// 0.45 skin h from where it was at the build.  A particle with more than
-// VL_CAP candidates records its rows' windows [start, end) instead, two to a
-// group, and tests every particle in them.
+// 0.45 skin h from where it was at the build.  A particle with more
+// candidates than the lists have room for records its rows' windows
+// [start, end) instead, two to a group, and tests every particle in them: two
+// to three times the candidates.  So the room follows the fluid at rest
+// (alloc_lists); with room for 96 at any packing and skin a step of 1,048,576
+// particles at h/2.6 and skin 0.2 took 1,347 us, now 532, and with one bit
+// mask per row, below, 589.
 //
 // Why flat lists: with one bit mask per stencil row the lanes of a warp wait
 // at every row for the one with most neighbours there (21 of 32 lanes active,
@@ -148,11 +152,19 @@ struct RowTables {
 // from slotScene (the .w lane of the sorted position, which carries the
 // scene in the batch's other kernels, holds p/rho^2 once a list density
 // kernel has run).
-constexpr int VL_GROUPS = 24;            // list groups of a particle
-constexpr int VL_CAP = 4 * VL_GROUPS;    // candidates they hold (~40 at the default skin in a fluid at rest)
+constexpr int VL_GROUPS_MIN = 24;        // list groups of a particle: at least (96 candidates) ...
+constexpr int VL_GROUPS_MAX = 96;        // ... and at most; alloc_lists chooses
+constexpr int VL_GROUPS_SHORT = 8;       // the fewest it falls back to where memory is short
+// Above this skin the density stage of a reusing step records which candidates
+// lie within h.  1,048,576 particles, force us without and with the masks: skin
+// 0.1 105 | 134, 0.2 154 | 137, 0.3 195 | 154, 0.4 202 | 154; with a packing of
+// h/2.6 0.1 257 | 302, 0.2 326 | 331.  (Only every second candidate is a
+// neighbour from 0.25 on, and a gather that is not made is worth the list
+// entries read one by one.)
+constexpr float VL_MASK_SKIN = 0.25f;
 constexpr int VL_ROWS = 16;              // rows within R <= 1.4 gridSpacing: at most 4 x 4
 constexpr unsigned int VL_WINDOWS = 0x80u;  // `groups` of a particle that records windows: this plus their number
-static_assert(VL_ROWS <= 2 * VL_GROUPS && VL_GROUPS < (int)VL_WINDOWS, "windows fit the groups");
+static_assert(VL_ROWS <= 2 * VL_GROUPS_SHORT && VL_GROUPS_MAX < (int)VL_WINDOWS, "windows fit the groups");
 enum : int {
     VL_BUILD = 0,      // a build is requested (state written, another kind of step ran)
     VL_BUILD_NOW = 1,  // this step's kind, a VL_REUSES ... (decided at the start of the step)
@@ -175,8 +187,11 @@ enum : unsigned int { VL_REUSES = 0, VL_BUILDS = 1, VL_SEARCHES = 2, VL_NOTHING 
 // from that step's sorted copies).
 enum : int { VL_SORT = 0, VL_STALE = 1, VL_GLOBAL = 2 };
 struct NeighbourLists {
-    int4* list;            // [VL_GROUPS][n] candidates within R, or two windows [start, end) a group
+    int4* list;            // [capacity][n] candidates within R, or two windows [start, end) a group
+    int capacity;          // groups allocated
     unsigned char* groups; // [n] groups in use, or VL_WINDOWS + windows in use
+    unsigned int* masks;   // [(capacity + 7) / 8][n] a reusing step's candidates within h, a bit each, eight
+                           //   groups a word; NULL: the force stage tests the candidates itself
     float4* posB;          // [n] positions at the build, working order
     unsigned int* flags;   // [VL_FLAGS][numScenes], then [VL_GLOBAL]
     float radius, radius2; // R and R^2 (single-scene handles; a batch's kernels take each scene's h)

@@ -159,7 +159,9 @@ void enqueue_step(sph_sim* s, int mode, bool timing, bool lists = true);
 // and the working order changed under them).
 void request_list_build(sph_sim* s);
 // Allocates the reused neighbour lists when the handle's options ask for them.
-sph_status alloc_lists(sph_sim* s);
+// How many candidates a particle inside the fluid at rest has on its list.
+double list_candidates(const PhysDev& ph, float skin);
+sph_status alloc_lists(sph_sim* s, double candidates);
 // Radius and displacement limit of the lists from the handle's parameters.
 void set_list_radius(sph_sim* s);
 // Hash, sort, density and force + integration (+ box collision) of the

@@ -192,7 +192,7 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
     auto append = [&](int t) {
         group = make_int4(group.y, group.z, group.w, t);
         count++;
-        if ((count & 3) == 0 && count <= VL_CAP) L.list[(size_t)((count >> 2) - 1) * n + i] = group;
+        if ((count & 3) == 0 && count <= 4 * L.capacity) L.list[(size_t)((count >> 2) - 1) * n + i] = group;
     };
     // every row the sphere reaches, in the reference's order (k outer, j inner)
     const int y1 = min(st.y1, st.y0 + 2), z1 = min(st.z1, st.z0 + 2);
@@ -255,7 +255,7 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
         M.start[at] = 0;
         M.mask[at] = 0u;
     }
-    if (lists && count <= VL_CAP) {
+    if (lists && count <= 4 * L.capacity) {
         L.groups[i] = (unsigned char)((count + 3) >> 2);
         while (count & 3) append(n);
     } else {
@@ -292,7 +292,7 @@ constexpr int DENSITY_LIST_BLOCKS = 4;
 // summed in plain FP32 (as a row's few terms are) and the group sums are
 // added with compensation.  The next group's slots are loaded before the
 // current group's positions are used.
-template <bool KAHAN, bool BATCH, bool FRESH>
+template <bool KAHAN, bool BATCH, bool MASKS, bool FRESH>
 __device__ __forceinline__ void density_list_one(int i, int n, float4* posS, float4* velS, const RowTables& T,
                                                  const GridDev& g, const PhysDev& ph_, const MapDev& map_,
                                                  float4* rho4S, const NeighbourLists& L, const RowMasks& M) {
@@ -316,14 +316,28 @@ __device__ __forceinline__ void density_list_one(int i, int n, float4* posS, flo
     if (!(groups & VL_WINDOWS)) {
         const int4* lp = L.list + i;
         int4 c = groups ? load_group<FRESH>(lp) : make_int4(0, 0, 0, 0);
+        unsigned int m = 0u;
 #pragma unroll 1
         for (unsigned int k = 0; k < groups; k++) {
             const float4 x0 = load<FRESH>(posS + c.x), x1 = load<FRESH>(posS + c.y), x2 = load<FRESH>(posS + c.z),
                          x3 = load<FRESH>(posS + c.w);
             lp += n;
             if (k + 1 < groups) c = load_group<FRESH>(lp);
-            const float w0 = fmaxf(h2 - dist2(xi, x0), 0.f), w1 = fmaxf(h2 - dist2(xi, x1), 0.f);
-            const float w2 = fmaxf(h2 - dist2(xi, x2), 0.f), w3 = fmaxf(h2 - dist2(xi, x3), 0.f);
+            const float r0 = dist2(xi, x0), r1 = dist2(xi, x1), r2 = dist2(xi, x2), r3 = dist2(xi, x3);
+            if (MASKS) {
+                unsigned int b = 0u;
+                if (neighbour_r2(r0, h2)) b = 1u;
+                if (neighbour_r2(r1, h2)) b |= 2u;
+                if (neighbour_r2(r2, h2)) b |= 4u;
+                if (neighbour_r2(r3, h2)) b |= 8u;
+                m |= b << (4 * (k & 7u));
+                if ((k & 7u) == 7u || k + 1 == groups) {
+                    L.masks[(size_t)(k >> 3) * n + i] = m;
+                    m = 0u;
+                }
+            }
+            const float w0 = fmaxf(h2 - r0, 0.f), w1 = fmaxf(h2 - r1, 0.f);
+            const float w2 = fmaxf(h2 - r2, 0.f), w3 = fmaxf(h2 - r3, 0.f);
             total(fmaf(w3 * w3, w3, fmaf(w2 * w2, w2, fmaf(w1 * w1, w1, w0 * w0 * w0))));
         }
     } else {
@@ -331,6 +345,7 @@ __device__ __forceinline__ void density_list_one(int i, int n, float4* posS, flo
         for (unsigned int w = 0; w < groups - VL_WINDOWS; w++) {
             const int2 se = list_window(L, n, i, (int)w);
             float rs = 0.f;
+#pragma unroll 4
             for (int t = se.x; t < se.y; t++) {
                 const float d = fmaxf(h2 - dist2(xi, load<FRESH>(posS + t)), 0.f);
                 rs = fmaf(d * d, d, rs);
@@ -353,12 +368,12 @@ __device__ __forceinline__ void density_list_one(int i, int n, float4* posS, flo
     velS[i].w = inv;
 }
 
-template <bool KAHAN, bool BATCH>
+template <bool KAHAN, bool BATCH, bool MASKS>
 __global__ void __launch_bounds__(256, DENSITY_LIST_BLOCKS)
 k_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDev g, PhysDev ph, MapDev map,
                 float4* __restrict__ rho4S, NeighbourLists L, RowMasks M) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) density_list_one<KAHAN, BATCH, false>(i, n, posS, velS, T, g, ph, map, rho4S, L, M);
+    if (i < n) density_list_one<KAHAN, BATCH, MASKS, false>(i, n, posS, velS, T, g, ph, map, rho4S, L, M);
 }
 
 // The far record: r^2 of any particle to it is ~3e36, beyond every support
@@ -838,13 +853,38 @@ __global__ void __launch_bounds__(256, FEAT ? 3 : (BATCH || TENSION || REL || FO
 // adds.  It also records, for the decision at the next step, the largest
 // squared distance of a particle from where it was when the lists were built.
 // ---------------------------------------------------------------------------
+// Which of the c <= 32 candidates from slot `base` on lie within h: a bit each.
+template <bool FRESH>
+__device__ __forceinline__ unsigned int row_hits(const float4* posS, int base, int c, float4 xi, float h2) {
+    unsigned int m = 0u;
+    const float4* p = posS + base;
+#pragma unroll 4
+    for (int k = 0; k < c; k++) m |= (neighbour_r2(dist2(xi, load<FRESH>(p + k)), h2) ? 1u : 0u) << k;
+    return m;
+}
+
 // The neighbours of a list step's particle: `pair` for each candidate (with
 // `tested` when it is known to lie within h), `row` with the sums of each
-// row's, window's or (group true) list group's pairs.
-template <bool TENSION, bool FRESH, class PAIR, class ROW>
+// row's, window's or (group true) list group's pairs.  MASKS: the density
+// stage has recorded which candidates lie within h, and only those are
+// gathered, four at a time too.
+template <bool TENSION, bool MASKS, bool FRESH, class PAIR, class ROW>
 __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const NeighbourLists& L, const RowMasks& M,
-                                          const float4* posS, const float4* velS,
+                                          const float4* posS, const float4* velS, float4 xi, float h2,
                                           PAIR&& pair, ROW&& row) {
+    // the pairs of the candidates [s, e): tested first, so that only the
+    // neighbours' velocities are loaded
+    auto range = [&](RowSums<TENSION>& R, int s, int e) {
+#pragma unroll 1
+        for (int base = s; base < e; base += 32) {
+            unsigned int m = row_hits<FRESH>(posS, base, min(32, e - base), xi, h2);
+            while (m) {
+                const int t = base + __ffs(m) - 1;
+                m &= m - 1u;
+                pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
+            }
+        }
+    };
     if (kind != VL_REUSES) {
         int svN = load<FRESH>(M.start + i);
         unsigned int mN = load<FRESH>(M.mask + i);
@@ -859,7 +899,7 @@ __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const
             RowSums<TENSION> R;
             R.clear();
             if (sv < 0) {
-                for (int t = sv & 0x7fffffff; t < (int)m; t++) pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), false);
+                range(R, sv & 0x7fffffff, (int)m);
             } else {
                 while (m) {
                     const int t = sv + __ffs(m) - 1;
@@ -878,8 +918,40 @@ __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const
             const int2 se = list_window(L, n, i, (int)w);
             RowSums<TENSION> R;
             R.clear();
-            for (int t = se.x; t < se.y; t++) pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), false);
+            range(R, se.x, se.y);
             row(R, false);
+        }
+        return;
+    }
+    if (MASKS) {
+#pragma unroll 1
+        for (unsigned int w = 0; 8 * w < groups; w++) {
+            unsigned int m = load<FRESH>(L.masks + (size_t)w * n + i);
+            const int* word = reinterpret_cast<const int*>(L.list + (size_t)(8 * w) * n + i);
+            auto next = [&]() {  // (past the last: the far record)
+                if (!m) return n;
+                const int k = __ffs(m) - 1;
+                m &= m - 1u;
+                return load<FRESH>(word + 4 * (size_t)(k >> 2) * n + (k & 3));
+            };
+            if (!m) continue;
+            int4 c = make_int4(next(), next(), next(), next());
+            while (c.x != n) {
+                const float4 x0 = load<FRESH>(posS + c.x), x1 = load<FRESH>(posS + c.y), x2 = load<FRESH>(posS + c.z), x3 = load<FRESH>(posS + c.w);
+                const float4 v0 = load<FRESH>(velS + c.x), v1 = load<FRESH>(velS + c.y), v2 = load<FRESH>(velS + c.z), v3 = load<FRESH>(velS + c.w);
+                const int4 d = c;
+                c.x = next();
+                c.y = next();
+                c.z = next();
+                c.w = next();
+                RowSums<TENSION> R;
+                R.clear();
+                pair(R, x0, v0, true);
+                if (d.y != n) pair(R, x1, v1, true);
+                if (d.z != n) pair(R, x2, v2, true);
+                if (d.w != n) pair(R, x3, v3, true);
+                row(R, true);
+            }
         }
         return;
     }
@@ -921,7 +993,7 @@ __device__ __forceinline__ void record_displacement(const NeighbourLists& L, int
 }
 
 // (every thread of the warp calls it: i may lie beyond the particles)
-template <bool KAHAN, bool TENSION, bool BATCH, bool FRESH>
+template <bool KAHAN, bool TENSION, bool BATCH, bool MASKS, bool FRESH>
 __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS, const float4* velS,
                                                const float4* rho4S, const int* workIds, const PhysDev& ph_,
                                                const MapDev& map_, int collideFlag, const NeighbourLists& L,
@@ -942,8 +1014,8 @@ __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS,
         ForceTotals<KAHAN, TENSION> A;
         // (a neighbour's p/rho^2 and 1/rho ride in the fourth lanes of its
         // sorted position and velocity, written by the density stage)
-        list_rows<TENSION, FRESH>(
-            i, n, kind, L, M, posS, velS,
+        list_rows<TENSION, MASKS, FRESH>(
+            i, n, kind, L, M, posS, velS, xi, h2,
             [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
                 Pair p(ph, xi, vi, xj, vj);
                 const bool in = tested || neighbour_r2(p.r2, h2);
@@ -980,13 +1052,13 @@ __device__ __forceinline__ void force_list_one(int i, int n, const float4* posS,
     record_displacement<BATCH>(L, scene, d2);
 }
 
-template <bool KAHAN, bool TENSION, bool BATCH>
+template <bool KAHAN, bool TENSION, bool BATCH, bool MASKS>
 __global__ void __maxnreg__(FORCE_REGS)
 k_force_lists(int n, const float4* __restrict__ posS, const float4* __restrict__ velS,
               const float4* __restrict__ rho4S, const int* __restrict__ workIds, PhysDev ph, MapDev map,
               int collideFlag, NeighbourLists L, RowMasks M, float4* __restrict__ pos, float4* __restrict__ vel,
               float4* __restrict__ accS, const SceneDev* __restrict__ scenes) {
-    force_list_one<KAHAN, TENSION, BATCH, false>(blockIdx.x * blockDim.x + threadIdx.x, n, posS, velS, rho4S, workIds,
+    force_list_one<KAHAN, TENSION, BATCH, MASKS, false>(blockIdx.x * blockDim.x + threadIdx.x, n, posS, velS, rho4S, workIds,
                                                  ph, map, collideFlag, L, M, pos, vel, accS, scenes);
 }
 
@@ -1033,7 +1105,7 @@ struct StepsArgs {
     int steps;
 };
 
-template <bool KAHAN, bool TENSION>
+template <bool KAHAN, bool TENSION, bool MASKS>
 __global__ void __launch_bounds__(STEPS_THREADS, STEPS_BLOCKS) k_steps(StepsArgs A) {
     const FrontArgs& F = A.F;
     unsigned int round = 0;
@@ -1047,11 +1119,11 @@ __global__ void __launch_bounds__(STEPS_THREADS, STEPS_BLOCKS) k_steps(StepsArgs
         barrier();
         if (!ok) break;
         for (int i = first; i < F.n; i += stride)
-            density_list_one<KAHAN, false, true>(i, F.n, F.posS, F.velS, A.T, F.g, A.ph, A.map, A.rho4S, F.L, A.M);
+            density_list_one<KAHAN, false, MASKS, true>(i, F.n, F.posS, F.velS, A.T, F.g, A.ph, A.map, A.rho4S, F.L, A.M);
         barrier();
         if (!ok) break;
         for (int base = blockIdx.x * STEPS_THREADS; base < F.n; base += stride)
-            force_list_one<KAHAN, TENSION, false, true>(base + (int)threadIdx.x, F.n, F.posS, F.velS, A.rho4S,
+            force_list_one<KAHAN, TENSION, false, MASKS, true>(base + (int)threadIdx.x, F.n, F.posS, F.velS, A.rho4S,
                                                         F.sb.workIds, A.ph, A.map, A.collide, F.L, A.M, A.pos, A.vel,
                                                         A.accS, nullptr);
         if (s + 1 < A.steps) barrier();
@@ -1253,7 +1325,7 @@ static_assert(L_BLOCKS_MAX * (L_SMEM + 1024) <= 227 * 1024 && L_BLOCKS_MAX * L_T
 // 1/rho from the fourth lanes of their sorted position and velocity, and the
 // kernel records the largest squared distance of a corrected position from where
 // the particle was when the lists were built.
-template <bool KAHAN, bool TENSION, int BLOCKS, bool LISTS>
+template <bool KAHAN, bool TENSION, int BLOCKS, bool LISTS, bool MASKS>
 __global__ void __launch_bounds__(L_THREADS, BLOCKS)
 k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
     using namespace mlp;
@@ -1301,8 +1373,8 @@ k_force_learned(ForceArgs F, MlpDev m, unsigned int* status, NeighbourLists L) {
             ForceTotals<KAHAN, TENSION> A;
             FeatSums fs;
             if (LISTS) {
-                list_rows<TENSION, false>(
-                    i, F.n, L.flags[VL_BUILD_NOW * L.numScenes], L, F.M, F.posS, F.velS,
+                list_rows<TENSION, MASKS, false>(
+                    i, F.n, L.flags[VL_BUILD_NOW * L.numScenes], L, F.M, F.posS, F.velS, xi, ph.h2,
                     [&](RowSums<TENSION>& R, float4 xj, float4 vj, bool tested) {
                         const Pair p(ph, xi, vi, xj, vj);
                         if (tested || neighbour_r2(p.r2, ph.h2)) {
@@ -1519,23 +1591,26 @@ void launch_force(int n, const float4* posS, const float4* velS, const float4* r
     }
 }
 
-template <bool KAHAN, bool TENSION, int BLOCKS, bool LISTS>
+template <bool KAHAN, bool TENSION, int BLOCKS, bool LISTS, bool MASKS = false>
 static void force_learned_launch(const ForceArgs& F, MlpDev m, unsigned int* status, const NeighbourLists& L,
                                  cudaStream_t s) {
-    ensure_dynamic_smem<k_force_learned<KAHAN, TENSION, BLOCKS, LISTS>>(L_SMEM);
-    k_force_learned<KAHAN, TENSION, BLOCKS, LISTS>
+    ensure_dynamic_smem<k_force_learned<KAHAN, TENSION, BLOCKS, LISTS, MASKS>>(L_SMEM);
+    k_force_learned<KAHAN, TENSION, BLOCKS, LISTS, MASKS>
         <<<(F.n + L_THREADS - 1) / L_THREADS, L_THREADS, L_SMEM, s>>>(F, m, status, L);
 }
 
-template <bool KAHAN, bool TENSION, bool LISTS>
-static void force_learned_dispatch(const ForceArgs& F, MlpDev m, unsigned int* status, const NeighbourLists& L,
+template <bool KAHAN, bool TENSION>
+static void force_learned_dispatch(const ForceArgs& F, MlpDev m, unsigned int* status, const NeighbourLists* L,
                                    cudaStream_t s) {
-    const int sms = device_sms();
     const long long blocks = (F.n + L_THREADS - 1) / L_THREADS;
-    if (!LISTS && blocks >= 2LL * L_BLOCKS_MAX * sms)
-        force_learned_launch<KAHAN, TENSION, L_BLOCKS_MAX, LISTS>(F, m, status, L, s);
+    if (L && L->masks)
+        force_learned_launch<KAHAN, TENSION, 3, true, true>(F, m, status, *L, s);
+    else if (L)
+        force_learned_launch<KAHAN, TENSION, 3, true>(F, m, status, *L, s);
+    else if (blocks >= 2LL * L_BLOCKS_MAX * device_sms())
+        force_learned_launch<KAHAN, TENSION, L_BLOCKS_MAX, false>(F, m, status, NeighbourLists{}, s);
     else
-        force_learned_launch<KAHAN, TENSION, 3, LISTS>(F, m, status, L, s);
+        force_learned_launch<KAHAN, TENSION, 3, false>(F, m, status, NeighbourLists{}, s);
 }
 
 void launch_force_learned(int n, const float4* posS, const float4* velS, const float4* rho4S, const int* workIds,
@@ -1547,21 +1622,14 @@ void launch_force_learned(int n, const float4* posS, const float4* velS, const f
     const FeatOut fo{feat.feat, feat.byId, feat.boxWalls, feat.dtL};
     ForceArgs F{n,  posS, velS, rho4S, workIds, T, g, ph, map, collide, cfg.prune,
                 RowMasks{const_cast<int*>(rowStart), const_cast<unsigned int*>(rowMask)}, pos, vel, accS, fo};
-    const NeighbourLists L = lists ? *lists : NeighbourLists{};
     const bool tension = ph.tension != 0.0f;
-#define SPH_FORCE_LEARNED(K, T)                                        \
-    do {                                                               \
-        if (lists) force_learned_dispatch<K, T, true>(F, m, status, L, s); \
-        else force_learned_dispatch<K, T, false>(F, m, status, L, s);      \
-    } while (0)
     if (cfg.kahan) {
-        if (tension) SPH_FORCE_LEARNED(true, true);
-        else SPH_FORCE_LEARNED(true, false);
+        if (tension) force_learned_dispatch<true, true>(F, m, status, lists, s);
+        else force_learned_dispatch<true, false>(F, m, status, lists, s);
     } else {
-        if (tension) SPH_FORCE_LEARNED(false, true);
-        else SPH_FORCE_LEARNED(false, false);
+        if (tension) force_learned_dispatch<false, true>(F, m, status, lists, s);
+        else force_learned_dispatch<false, false>(F, m, status, lists, s);
     }
-#undef SPH_FORCE_LEARNED
 }
 
 // After the positions were written: the largest squared distance of a
@@ -1596,14 +1664,18 @@ void launch_density_lists(int n, float4* posS, float4* velS, RowTables T, GridDe
     if (n <= 0) return;
     const int bs = cfg.densityBlock > 0 ? cfg.densityBlock : 128;
     const int grid = (n + bs - 1) / bs;
-#define SPH_DENSITY_LISTS(K, B) k_density_lists<K, B><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L, M)
-    if (cfg.kahan) {
-        if (T.scenes) SPH_DENSITY_LISTS(true, true);
-        else SPH_DENSITY_LISTS(true, false);
-    } else {
-        if (T.scenes) SPH_DENSITY_LISTS(false, true);
-        else SPH_DENSITY_LISTS(false, false);
-    }
+#define SPH_DENSITY_LISTS(K, B, X) \
+    k_density_lists<K, B, X><<<grid, bs, 0, s>>>(n, posS, velS, T, g, ph, map, rho4S, L, M)
+#define SPH_DENSITY_LISTS_B(K)                                \
+    do {                                                      \
+        if (T.scenes && L.masks) SPH_DENSITY_LISTS(K, true, true); \
+        else if (T.scenes) SPH_DENSITY_LISTS(K, true, false); \
+        else if (L.masks) SPH_DENSITY_LISTS(K, false, true);  \
+        else SPH_DENSITY_LISTS(K, false, false);              \
+    } while (0)
+    if (cfg.kahan) SPH_DENSITY_LISTS_B(true);
+    else SPH_DENSITY_LISTS_B(false);
+#undef SPH_DENSITY_LISTS_B
 #undef SPH_DENSITY_LISTS
 }
 
@@ -1616,13 +1688,15 @@ void launch_force_lists(int n, const float4* posS, const float4* velS, const flo
     // (a batch's tension coefficient is the largest of its scenes': it selects
     // whether the colour field is computed at all)
     const bool tension = ph.tension != 0.0f;
-#define SPH_FORCE_LISTS(K, T, B)                                                                             \
-    k_force_lists<K, T, B><<<grid, bs, 0, s>>>(n, posS, velS, rho4S, workIds, ph, map, collide, L, M, pos, vel, \
-                                               accS, scenes)
-#define SPH_FORCE_LISTS_B(K, T)           \
-    do {                                  \
-        if (scenes) SPH_FORCE_LISTS(K, T, true);  \
-        else SPH_FORCE_LISTS(K, T, false);        \
+#define SPH_FORCE_LISTS(K, T, B, X)                                                                             \
+    k_force_lists<K, T, B, X><<<grid, bs, 0, s>>>(n, posS, velS, rho4S, workIds, ph, map, collide, L, M, pos, vel, \
+                                                  accS, scenes)
+#define SPH_FORCE_LISTS_B(K, T)                                \
+    do {                                                       \
+        if (scenes && L.masks) SPH_FORCE_LISTS(K, T, true, true); \
+        else if (scenes) SPH_FORCE_LISTS(K, T, true, false);   \
+        else if (L.masks) SPH_FORCE_LISTS(K, T, false, true);  \
+        else SPH_FORCE_LISTS(K, T, false, false);              \
     } while (0)
     if (cfg.kahan) {
         if (tension) SPH_FORCE_LISTS_B(true, true);
@@ -1635,12 +1709,12 @@ void launch_force_lists(int n, const float4* posS, const float4* velS, const flo
 #undef SPH_FORCE_LISTS
 }
 
-template <bool KAHAN, bool TENSION>
+template <bool KAHAN, bool TENSION, bool MASKS>
 static void steps_launch(StepsArgs& A, cudaStream_t s) {
     const int want = std::max((A.F.n + STEPS_THREADS - 1) / STEPS_THREADS, A.F.g.numCells / (16 * STEPS_THREADS));
-    const int grid = std::min(want, resident_blocks<k_steps<KAHAN, TENSION>>(STEPS_THREADS, STEPS_BLOCKS));
+    const int grid = std::min(want, resident_blocks<k_steps<KAHAN, TENSION, MASKS>>(STEPS_THREADS, STEPS_BLOCKS));
     void* args[] = {&A};
-    cudaLaunchCooperativeKernel((const void*)k_steps<KAHAN, TENSION>, dim3(grid), dim3(STEPS_THREADS), args, 0, s);
+    cudaLaunchCooperativeKernel((const void*)k_steps<KAHAN, TENSION, MASKS>, dim3(grid), dim3(STEPS_THREADS), args, 0, s);
 }
 
 bool takes_whole_steps(int n, int numCells) { return n <= STEPS_PARTICLES && numCells <= STEPS_CELLS; }
@@ -1654,13 +1728,19 @@ void launch_steps(int n, float4* pos, float4* vel, GridDev g, SortBuffers sb, Ro
     const bool tension = ph.tension != 0.0f;
     for (; steps > 0; steps -= A.steps) {
         A.steps = std::min(steps, STEPS_A_LAUNCH);
+#define SPH_STEPS(K, T)                          \
+    do {                                         \
+        if (L.masks) steps_launch<K, T, true>(A, s); \
+        else steps_launch<K, T, false>(A, s);    \
+    } while (0)
         if (cfg.kahan) {
-            if (tension) steps_launch<true, true>(A, s);
-            else steps_launch<true, false>(A, s);
+            if (tension) SPH_STEPS(true, true);
+            else SPH_STEPS(true, false);
         } else {
-            if (tension) steps_launch<false, true>(A, s);
-            else steps_launch<false, false>(A, s);
+            if (tension) SPH_STEPS(false, true);
+            else SPH_STEPS(false, false);
         }
+#undef SPH_STEPS
     }
 }
 
