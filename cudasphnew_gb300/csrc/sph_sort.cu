@@ -198,7 +198,11 @@ static void front_launch(FrontArgs A, cudaStream_t s) {
     const long long want = std::max(((long long)A.n + FRONT_THREADS - 1) / FRONT_THREADS,
                                     ((long long)A.g.numCells + 16 * FRONT_THREADS) / (16 * FRONT_THREADS));
     const int most = resident_blocks<k_front<BATCH, REL>>(FRONT_THREADS, A.n > FRONT_WIDE ? 2 : 1);
-    const int grid = (int)std::max(1ll, std::min(want, (long long)most));
+    // no more blocks than the last of their passes over the particles fills:
+    // the SMs they leave are other handles' (six, searching, in turn: 131,072
+    // particles 40.1 -> 39.2 us a step, 98,304 31.8 -> 29.3; one alone the same)
+    const long long passes = (want + most - 1) / most;
+    const int grid = (int)std::max(1ll, (want + passes - 1) / passes);
     void* args[] = {&A};
     cudaLaunchCooperativeKernel((const void*)k_front<BATCH, REL>, dim3(grid), dim3(FRONT_THREADS), args, 0, s);
 }

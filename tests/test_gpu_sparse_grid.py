@@ -22,11 +22,7 @@ def scattered(side, n, skin):
     return scenes.Scene("sparse", p, o, x.astype(np.float32), np.zeros((n, 3), np.float32))
 
 
-# cells a side: 8 .. 244 (14.5 million cells)
-@pytest.mark.parametrize("side", [0.1, 0.15, 0.2, 0.5, 1.0, 1.6, 3.0, 6.0])
-@pytest.mark.parametrize("n, skin", [(700, 0.0), (700, 0.1), (30000, 0.0), (30000, 0.1)])
-def test_cell_tables_of_sparse_grids(sphlib, side, n, skin):
-    sc = scattered(side, n, skin)
+def check_cells(sphlib, sc):
     g = sc.params
     dim = [int(d) for d in g.gridDim]
     with sphlib.ParticleSimulation(g, sc.positions, None, sc.options) as sim:
@@ -46,3 +42,16 @@ def test_cell_tables_of_sparse_grids(sphlib, side, n, skin):
             empty = np.ones(len(start), bool)
             empty[cells] = False
             assert (start[empty] == start[empty][0]).all() and (end[empty] == end[empty][0]).all()
+
+
+# cells a side: 8 .. 244 (14.5 million cells)
+@pytest.mark.parametrize("side", [0.1, 0.15, 0.2, 0.5, 1.0, 1.6, 3.0, 6.0])
+@pytest.mark.parametrize("n, skin", [(700, 0.0), (700, 0.1), (30000, 0.0), (30000, 0.1)])
+def test_cell_tables_of_sparse_grids(sphlib, side, n, skin):
+    check_cells(sphlib, scattered(side, n, skin))
+
+
+# one, two and three passes of a block an SM (152) of 512 particles, and one particle more
+@pytest.mark.parametrize("n", [77824, 77825, 155648, 155649, 233472, 233473])
+def test_cell_tables_where_the_grid_takes_another_pass(sphlib, n):
+    check_cells(sphlib, scattered(1.0, n, 0.0))
