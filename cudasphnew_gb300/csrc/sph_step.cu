@@ -1089,7 +1089,7 @@ constexpr int STEPS_PARTICLES = 24576;
 constexpr int STEPS_CELLS = 1 << 18;
 constexpr int STEPS_BLOCKS = 4;  // blocks an SM (128 registers a thread: no spills)
 constexpr int STEPS_THREADS = 128;
-constexpr int STEPS_A_LAUNCH = 32;  // (a bound on a launch: half a millisecond)
+constexpr int STEPS_A_LAUNCH = 32;  // (a bound on a launch: 0.74 ms for 24,576 particles that reuse their lists)
 
 struct StepsArgs {
     FrontArgs F;

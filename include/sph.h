@@ -279,8 +279,9 @@ sph_status sph_set_stream(sph_handle h, void* stream);
 sph_status sph_step(sph_handle h, int mode);
 
 /* Enqueues `count` steps of `mode` (one CUDA-graph launch each once captured;
- * plain steps of a handle with reused lists and at most 24,576 particles: up
- * to 32 in one launch).  The results are those of `count` calls of sph_step. */
+ * plain steps of a handle with reused lists, at most 24,576 particles and at
+ * most 2^18 cells: up to 32 in one launch).  The results are those of `count`
+ * calls of sph_step.  Refused on a stream that is being captured. */
 sph_status sph_step_many(sph_handle h, int mode, int count);
 
 /* Waits for the handle's stream; returns the latched device status. */
@@ -545,7 +546,11 @@ sph_status sph_set_tuning(sph_handle h, const sph_tuning* t);
 /* Times every candidate launch configuration of the density and force
  * kernels on the handle's current particle state (`reps` launches each, CUDA
  * events on the handle's stream), keeps the fastest and returns it.  The
- * simulation state is left untouched.  No reference counterpart. */
+ * simulation state is left untouched.  (The plain steps of a handle that
+ * takes whole steps in one launch, see sph_step_many, have no block sizes to
+ * choose; its stages do where they run on their own, in learned and
+ * stage-timed steps, and take the same time at each of them.)  No reference
+ * counterpart. */
 sph_status sph_autotune(sph_handle h, int reps, sph_tuning* chosen);
 
 /* Stage timing with CUDA events on the handle's stream (CudaTimer,
@@ -566,7 +571,8 @@ const char* sph_stage_name(int stage);
 /* Average device time of one launch of a stage's kernel (stage 4: density,
  * 5: force; see sph_stage_name), launched `reps` times back to back on the
  * last step's sorted state between two CUDA events on the handle's stream,
- * with the current tuning.  Both kernels rewrite what they wrote: after a
+ * with the current tuning (the stage's own kernel also on a handle whose plain
+ * steps are single launches).  Both kernels rewrite what they wrote: after a
  * plain step the force stage leaves the state that step left (after another
  * kind of step it replaces that step's result with the plain step's).  No
  * reference counterpart. */
