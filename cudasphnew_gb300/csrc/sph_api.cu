@@ -183,7 +183,7 @@ void free_all(sph_sim* s) {
                     s->sb.keySlot, s->sb.tmpIds, s->sb.sortedHash, s->sb.sortedIds, s->sb.workIds,
                     s->sb.halfOffset, s->sb.front,
                     s->status, s->staging, s->map4, s->mapDist, s->rowStart, s->rowMask, s->diagBuf,
-                    s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.masks, s->vl.posB,
+                    s->scenesDev, s->reuse, s->vl.list, s->vl.groups, s->vl.rowMask2, s->vl.masks, s->vl.posB,
                     s->vl.flags, s->vl.slotScene};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -312,14 +312,13 @@ double list_candidates(const PhysDev& ph, float skin) {
     return std::isfinite(inside) ? inside : 0.0;
 }
 
-// (room for twice the candidates of a particle inside the fluid at rest, so
-// that only a fluid compressed to twice its density records windows)
 sph_status alloc_lists(sph_sim* s, double candidates) {
     if (!(s->O.neighbourSkin > 0.0f) || s->O.cellRelative) return SPH_OK;
     const size_t n = (size_t)s->n;
     const int S = std::max(s->numScenes, 1);
     SPH_CUDA(dalloc(&s->vl.groups, n));
     SPH_CUDA(dalloc(&s->vl.posB, n));
+    SPH_CUDA(dalloc(&s->vl.rowMask2, 9 * n));
     SPH_CUDA(dalloc(&s->vl.flags, (size_t)VL_FLAGS * S + VL_GLOBAL));
     SPH_CUDA(cudaMemsetAsync(s->vl.flags, 0, sizeof(unsigned int) * (VL_FLAGS * S + VL_GLOBAL), s->stream));
     s->vl.numScenes = S;
@@ -332,8 +331,13 @@ sph_status alloc_lists(sph_sim* s, double candidates) {
         SPH_CUDA(dalloc(&s->vl.slotScene, n));
         SPH_CUDA(cudaMemcpy(s->vl.slotScene, scene.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     }
-    s->vl.capacity = (int)std::min(std::max(std::ceil(2.0 * candidates / 4.0), (double)VL_GROUPS_MIN),
-                                   (double)VL_GROUPS_MAX);
+    // as much room as a sixteenth of the free memory gives, but always for
+    // twice the candidates of a particle inside the fluid at rest
+    size_t freeBytes = 0, allBytes = 0;
+    SPH_CUDA(cudaMemGetInfo(&freeBytes, &allBytes));
+    const double room = (double)freeBytes / 16.0 / ((double)sizeof(int4) * (double)n);
+    const double need = std::max(std::ceil(2.0 * candidates / 4.0), (double)VL_GROUPS_MIN);
+    s->vl.capacity = (int)std::min(std::max(room, need), (double)VL_GROUPS_MAX);
     // (where memory is short, fewer groups: more particles record windows)
     cudaError_t e = dalloc(&s->vl.list, (size_t)s->vl.capacity * n);
     while (e == cudaErrorMemoryAllocation && s->vl.capacity > VL_GROUPS_SHORT) {

@@ -136,10 +136,13 @@ struct RowTables {
 // 0.45 skin h from where it was at the build.  A particle with more
 // candidates than the lists have room for records its rows' windows
 // [start, end) instead, two to a group, and tests every particle in them: two
-// to three times the candidates.  So the room follows the fluid at rest
-// (alloc_lists); with room for 96 at any packing and skin a step of 1,048,576
-// particles at h/2.6 and skin 0.2 took 1,347 us, now 532, and with one bit
-// mask per row, below, 589.
+// to three times the candidates.  The fluid is soft and its lower layers
+// compress, a particle there has three to eight times the candidates of one at
+// rest (44 at the default skin), so the lists take all the room there is
+// (alloc_lists).  With room for 96 a step of the 1,048,576-particle obstacle
+// scene took 235 us after 500 steps, 636 after 2,000 and 2,131 after 4,000,
+// now 235, 441 and 1,747; with one bit mask per row, below, 290, 509 and 1,710
+// (there every tenth particle of the fluid has 355 candidates or more).
 //
 // Why flat lists: with one bit mask per stencil row the lanes of a warp wait
 // at every row for the one with most neighbours there (21 of 32 lanes active,
@@ -153,7 +156,7 @@ struct RowTables {
 // scene in the batch's other kernels, holds p/rho^2 once a list density
 // kernel has run).
 constexpr int VL_GROUPS_MIN = 24;        // list groups of a particle: at least (96 candidates) ...
-constexpr int VL_GROUPS_MAX = 96;        // ... and at most; alloc_lists chooses
+constexpr int VL_GROUPS_MAX = 120;       // ... and at most; alloc_lists chooses
 constexpr int VL_GROUPS_SHORT = 8;       // the fewest it falls back to where memory is short
 // Above this skin the density stage of a reusing step records which candidates
 // lie within h.  1,048,576 particles, force us without and with the masks: skin
@@ -190,6 +193,7 @@ struct NeighbourLists {
     int4* list;            // [capacity][n] candidates within R, or two windows [start, end) a group
     int capacity;          // groups allocated
     unsigned char* groups; // [n] groups in use, or VL_WINDOWS + windows in use
+    unsigned int* rowMask2; // [9][n] of RowMasks' rows with 33 to 64 places: the bits of the upper half
     unsigned int* masks;   // [(capacity + 7) / 8][n] a reusing step's candidates within h, a bit each, eight
                            //   groups a word; NULL: the force stage tests the candidates itself
     float4* posB;          // [n] positions at the build, working order
@@ -203,11 +207,13 @@ struct NeighbourLists {
 };
 
 // What the density stage records for the force stage of the per-step search,
-// and of a step that builds the lists.
+// and of a step that builds the lists (there also rows of 33 to 64 places,
+// ROW_TWO_WORDS set in their start: NeighbourLists::rowMask2).
 struct RowMasks {
     int* start;          // [9][n] window start, bit 31 set when the row was not masked
     unsigned int* mask;  // [9][n] neighbour bits relative to start, or the window end
 };
+constexpr int ROW_TWO_WORDS = 0x40000000;  // (a handle's particles are fewer: 2^30 would take 400 GB)
 
 // Launch configuration of the step (chosen per handle; see the autotuner).
 enum ForceVariant { FORCE_DIRECT = 0, FORCE_MASK = 1, FORCE_PRETESTED = 2, FORCE_STAGED = 3 };

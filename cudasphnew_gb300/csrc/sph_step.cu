@@ -217,7 +217,7 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
         const bool inner = z >= st.z0 && z <= z1 && y >= st.y0 && y <= y1;
         float rs = 0.f;
         int first = -1, last = -1;
-        unsigned int m = 0u;  // neighbours within h, bit t - first
+        unsigned long long m = 0ull;  // neighbours within h, bit t - first
         for (int base = s0; base < e0; base += 32) {
             unsigned int mR, mh;
             row_tests<false, true, FRESH>(posS, base, min(32, e0 - base), xi, h2, R2, 0, 0.f, 0.f, 0.f, rs, mR, mh);
@@ -226,8 +226,8 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
                     const int k = __ffs(mh) - 1;
                     first = base + k;
                     m = mh >> k;
-                } else if (base - first < 32) {
-                    m |= mh << (base - first);
+                } else if (base - first < 64) {
+                    m |= (unsigned long long)mh << (base - first);
                 }
                 last = base + 31 - __clz(mh);
             }
@@ -244,11 +244,13 @@ __device__ __forceinline__ void density_build_one(int i, int n, bool lists, int 
         } else {
             sum += rs;
         }
-        const bool fits = last - first < 32;
+        const int places = last - first + 1;
         const int slot = 3 * (z - st.z0) + y - st.y0;
+        const size_t at = (size_t)slot * n + i;
         seen |= 1u << slot;
-        M.start[(size_t)slot * n + i] = first < 0 ? 0 : fits ? first : (first | (int)0x80000000);
-        M.mask[(size_t)slot * n + i] = fits ? m : (unsigned int)(last + 1);
+        M.start[at] = first < 0 ? 0 : places <= 32 ? first : first | (places <= 64 ? ROW_TWO_WORDS : (int)0x80000000);
+        M.mask[at] = places <= 64 ? (unsigned int)m : (unsigned int)(last + 1);
+        if (places > 32 && places <= 64) L.rowMask2[at] = (unsigned int)(m >> 32);
     });
     for (unsigned int none = ~seen & 0x1ffu; none; none &= none - 1u) {
         const size_t at = (size_t)(__ffs(none) - 1) * n + i;
@@ -858,8 +860,19 @@ template <bool FRESH>
 __device__ __forceinline__ unsigned int row_hits(const float4* posS, int base, int c, float4 xi, float h2) {
     unsigned int m = 0u;
     const float4* p = posS + base;
-#pragma unroll 4
-    for (int k = 0; k < c; k++) m |= (neighbour_r2(dist2(xi, load<FRESH>(p + k)), h2) ? 1u : 0u) << k;
+    int k = 0;
+#pragma unroll 1
+    for (; k + 4 <= c; k += 4, p += 4) {
+        const float4 x0 = load<FRESH>(p), x1 = load<FRESH>(p + 1), x2 = load<FRESH>(p + 2), x3 = load<FRESH>(p + 3);
+        unsigned int b = 0u;
+        if (neighbour_r2(dist2(xi, x0), h2)) b = 1u;
+        if (neighbour_r2(dist2(xi, x1), h2)) b |= 2u;
+        if (neighbour_r2(dist2(xi, x2), h2)) b |= 4u;
+        if (neighbour_r2(dist2(xi, x3), h2)) b |= 8u;
+        m |= b << k;
+    }
+#pragma unroll 1
+    for (; k < c; k++, p++) m |= (neighbour_r2(dist2(xi, load<FRESH>(p)), h2) ? 1u : 0u) << k;
     return m;
 }
 
@@ -901,10 +914,17 @@ __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const
             if (sv < 0) {
                 range(R, sv & 0x7fffffff, (int)m);
             } else {
-                while (m) {
-                    const int t = sv + __ffs(m) - 1;
-                    m &= m - 1u;
-                    pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
+                auto bits = [&](int base) {
+                    while (m) {
+                        const int t = base + __ffs(m) - 1;
+                        m &= m - 1u;
+                        pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
+                    }
+                };
+                bits(sv & ~ROW_TWO_WORDS);
+                if (sv & ROW_TWO_WORDS) {
+                    m = load<FRESH>(L.rowMask2 + (size_t)r * n + i);
+                    bits((sv & ~ROW_TWO_WORDS) + 32);
                 }
             }
             row(R, false);
