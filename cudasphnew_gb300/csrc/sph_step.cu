@@ -885,47 +885,50 @@ template <bool TENSION, bool MASKS, bool FRESH, class PAIR, class ROW>
 __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const NeighbourLists& L, const RowMasks& M,
                                           const float4* posS, const float4* velS, float4 xi, float h2,
                                           PAIR&& pair, ROW&& row) {
-    // the pairs of the candidates [s, e): tested first, so that only the
-    // neighbours' velocities are loaded
-    auto range = [&](RowSums<TENSION>& R, int s, int e) {
+    // the pairs of `places` places from `base` on, 32 at a time: m holds the
+    // neighbours among the first, more(base, places) those of the next
+    auto walk = [&](RowSums<TENSION>& R, int base, int places, unsigned int m, auto&& more) {
 #pragma unroll 1
-        for (int base = s; base < e; base += 32) {
-            unsigned int m = row_hits<FRESH>(posS, base, min(32, e - base), xi, h2);
+        for (;;) {
             while (m) {
                 const int t = base + __ffs(m) - 1;
                 m &= m - 1u;
                 pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
             }
+            places -= 32;
+            if (places <= 0) break;
+            base += 32;
+            m = more(base, min(32, places));
         }
     };
+    // (tested first, so that only the neighbours' velocities are loaded)
+    auto hits = [&](int base, int places) { return row_hits<FRESH>(posS, base, places, xi, h2); };
     if (kind != VL_REUSES) {
         int svN = load<FRESH>(M.start + i);
         unsigned int mN = load<FRESH>(M.mask + i);
 #pragma unroll 1
         for (int r = 0; r < 9; r++) {
             const int sv = svN;
-            unsigned int m = mN;
+            const unsigned int m = mN;
             if (r + 1 < 9) {
                 svN = load<FRESH>(M.start + (size_t)(r + 1) * n + i);
                 mN = load<FRESH>(M.mask + (size_t)(r + 1) * n + i);
             }
             RowSums<TENSION> R;
             R.clear();
-            if (sv < 0) {
-                range(R, sv & 0x7fffffff, (int)m);
-            } else {
-                auto bits = [&](int base) {
-                    while (m) {
-                        const int t = base + __ffs(m) - 1;
-                        m &= m - 1u;
-                        pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
-                    }
-                };
-                bits(sv & ~ROW_TWO_WORDS);
-                if (sv & ROW_TWO_WORDS) {
-                    m = load<FRESH>(L.rowMask2 + (size_t)r * n + i);
-                    bits((sv & ~ROW_TWO_WORDS) + 32);
+            if ((unsigned int)sv < (unsigned int)ROW_TWO_WORDS) {
+                unsigned int b = m;
+                while (b) {
+                    const int t = sv + __ffs(b) - 1;
+                    b &= b - 1u;
+                    pair(R, load<FRESH>(posS + t), load<FRESH>(velS + t), true);
                 }
+            } else {
+                const int base = sv & ~((int)0x80000000 | ROW_TWO_WORDS);
+                const int places = sv < 0 ? (int)m - base : 64;
+                walk(R, base, places, sv < 0 ? hits(base, 32) : m, [&](int b, int c) {
+                    return sv < 0 ? hits(b, c) : load<FRESH>(L.rowMask2 + (size_t)r * n + i);
+                });
             }
             row(R, false);
         }
@@ -938,7 +941,7 @@ __device__ __forceinline__ void list_rows(int i, int n, unsigned int kind, const
             const int2 se = list_window(L, n, i, (int)w);
             RowSums<TENSION> R;
             R.clear();
-            range(R, se.x, se.y);
+            walk(R, se.x, se.y - se.x, hits(se.x, min(32, se.y - se.x)), hits);
             row(R, false);
         }
         return;
