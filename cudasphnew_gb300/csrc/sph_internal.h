@@ -141,7 +141,7 @@ struct RowTables {
 // rest (44 at the default skin), so the lists take all the room there is
 // (alloc_lists).  With room for 96 a step of the 1,048,576-particle obstacle
 // scene took 235 us after 500 steps, 636 after 2,000 and 2,131 after 4,000,
-// now 235, 441 and 1,747; with one bit mask per row, below, 290, 509 and 1,710
+// now 236, 451 and 1,708; with one bit mask per row, below, 290, 509 and 1,710
 // (there every tenth particle of the fluid has 355 candidates or more).
 //
 // Why flat lists: with one bit mask per stencil row the lanes of a warp wait

@@ -114,7 +114,12 @@ typedef struct sph_options {
                             neighbour sums are taken follows the lists.  Lists
                             are not built where the step before, by its own
                             motion, has outrun those just built: such a step
-                            searches as with 0, until the motion slows.  0: the
+                            searches as with 0, until the motion slows.  The
+                            lists take up to 1,920 bytes of device memory a
+                            particle, within a sixteenth of what is free when
+                            the handle is created (but 384 where they can be
+                            had); particles with more candidates than fit test
+                            all particles of their rows' windows.  0: the
                             neighbour search runs in every step, as the
                             reference does (compute_particle_density_pressure,
                             :196-256).  In [0, 0.4].  No reference counterpart. */
